@@ -113,6 +113,7 @@ struct Context
     // nothing
     long long tab_nmax[TAB_SLOTS] = {-1, -1, -1};
     unsigned long long tab_used[TAB_SLOTS] = {};
+    bool tab_two[TAB_SLOTS] = {};   // the slot's two-degree tables are built
     unsigned long long tab_clock = 0;
     // bumped whenever a cached device buffer is (re)allocated or a cached
     // table is rewritten: a captured graph reads these by address, so it
@@ -127,8 +128,8 @@ struct Context
     bool capturing = false;
     std::vector<void *> capture_pins;
     // autotuned latitude pairs per lane of the synthesis kernel, per
-    // (kgrad, dr, dlat, r != R, nmax, pairs); value and the measured ms of
-    // each candidate
+    // (kgrad, dr, dlat, kernel variant, nmax, pairs); value and the measured
+    // ms of each candidate
     std::map<std::tuple<int, int, int, int, long long, int>,
              std::pair<int, std::vector<std::pair<int, float>>>>
         tuned;
@@ -640,6 +641,10 @@ void host_smm(long long nmax, double *smm)
     }
 }
 
+// Steps of the two-degree recurrence over all orders of degree nmax
+// (two_sum of two.cuh).
+long long two_steps(long long nmax) { return ((nmax + 2) * (nmax + 2)) / 4; }
+
 // Recurrence tables of the rescaled recurrence (leg.cuh, tables.cu), built
 // once per maximum degree and kept on the device.
 struct Tabs
@@ -650,9 +655,12 @@ struct Tabs
     int ldmul = 0;
     double *sg = nullptr;
     double *dm = nullptr;
+    // two-degree recurrence (two.cuh), with two = true only
+    double2 *ab = nullptr, *ag = nullptr;
+    double *kw = nullptr, *sm = nullptr;
 };
 
-Status tables(Context &c, long long nmax, Tabs *tab)
+Status tables(Context &c, long long nmax, Tabs *tab, bool two = false)
 {
     Status st;
     long long T = (nmax + 1) * (nmax + 2) / 2;
@@ -677,10 +685,33 @@ Status tables(Context &c, long long nmax, Tabs *tab)
                 &tab->tmul));
     CB_TRY(dbuf(c, "tab_sg" + sfx, (size_t)(2 * (nmax + 1)), &tab->sg));
     CB_TRY(dbuf(c, "tab_dm" + sfx, (size_t)(nmax + 1), &tab->dm));
+    if (!hit)
+    {
+        // the slot is rewritten: invalid until the rebuild below completes
+        c.tab_nmax[slot] = -1;
+        c.tab_two[slot] = false;
+    }
+    if (two)
+    {
+        const size_t TL = (size_t)two_steps(nmax);
+        CB_TRY(dbuf(c, "tab_ab" + sfx, TL, &tab->ab));
+        CB_TRY(dbuf(c, "tab_ag" + sfx, TL, &tab->ag));
+        CB_TRY(dbuf(c, "tab_kw" + sfx, 3 * TL, &tab->kw));
+        CB_TRY(dbuf(c, "tab_sm" + sfx, (size_t)(nmax + 1), &tab->sm));
+    }
+    auto build_two = [&]() -> Status {
+        Status s2;
+        if (!two || c.tab_two[slot])
+            return s2;
+        c.epoch++;
+        Scope sc(c, TIMER_TABLES);
+        CB_CUDA(launch_two_tables(nmax, tab->sg, tab->ab, tab->ag, tab->kw,
+                                  tab->sm, c.stream), s2);
+        c.tab_two[slot] = true;
+        return s2;
+    };
     if (hit)
-        return st;
-    // the slot is rewritten: invalid until the rebuild below completes
-    c.tab_nmax[slot] = -1;
+        return build_two();
     c.epoch++;
     std::vector<double> r, ri, dmh;
     host_r_ri_dm(nmax, r, ri, dmh);
@@ -703,6 +734,7 @@ Status tables(Context &c, long long nmax, Tabs *tab)
         CB_CUDA(launch_tables(nmax, dr, dri, dsm, tab->tb, tab->tc, tab->tmul,
                               tab->ldmul, tab->sg, c.stream), st);
     }
+    CB_TRY(build_two());
     // the host vectors must outlive the copies
     CB_CUDA(cudaStreamSynchronize(c.stream), st);
     c.tab_nmax[slot] = nmax;
@@ -1184,6 +1216,29 @@ int choose_k(int kgrad, int dlat, long long nunits)
     return nunits >= 64 ? 2 : 1;
 }
 
+// Latitude pairs per lane of the two-degree synthesis (shs_two.cu) where the
+// autotuner does not run: for many latitudes the width of least padding
+// among 4..6 (the fastest three at nmax 2190 and 5400, within 4% of one
+// another), 15 K + 6 issue cycles per step; narrow tiles for few latitudes,
+// where the items of wide ones would not fill the GPU (K = 1 fastest at 181
+// and 251 pairs, 2 at 501 and 721).
+int choose_k_two(int n2)
+{
+    if (n2 <= 896)
+        return n2 >= 320 ? 2 : 1;
+    int best = 4, cost = 0;
+    for (int k = 4; k <= 6; k++)
+    {
+        const int t = (n2 + 32 * k - 1) / (32 * k) * (15 * k + 6);
+        if (cost == 0 || t < cost)
+        {
+            cost = t;
+            best = k;
+        }
+    }
+    return best;
+}
+
 // Latitude pairs per lane of the analysis kernel.  Wider tiles amortise
 // the per-degree beta load and the transpose-reduce over more latitudes but
 // lower the resident warps (sha_grid.cu); CHARM_B200_SHA_K (1, 2, 4, 6 or
@@ -1222,57 +1277,47 @@ bool autotune_on()
 // True when tune_shs_k launches nothing for this shape (tuned already, or
 // not tuned at all), so that the call's coefficients need not all be on
 // the device before its first synthesis launch.
-bool shs_k_settled(Context &c, int kgrad, int dr, int dlat, bool rr,
+bool shs_k_settled(Context &c, int kgrad, int dr, int dlat, int variant,
                    long long nmax, int np)
 {
-    const auto key = std::make_tuple(kgrad, dr, dlat, rr ? 1 : 0, nmax, np);
+    const auto key = std::make_tuple(kgrad, dr, dlat, variant, nmax, np);
     return c.tuned.count(key) > 0 || !autotune_on() || nmax < 256;
 }
 
-Status tune_shs_k(Context &c, const ShsGridArgs &A0, int kgrad, int dr,
-                  int dlat, bool rr, int np, int *K)
+// launch(K) runs the call's synthesis with K pairs per lane (its counter
+// cleared); cands: the widths to time, besides the built-in *K.
+template <typename F>
+Status tune_shs_k(Context &c, const F &launch, std::vector<int> cands,
+                  int kgrad, int dr, int dlat, int variant, long long nmax,
+                  int np, int *K)
 {
     Status st;
-    const auto key = std::make_tuple(kgrad, dr, dlat, rr ? 1 : 0, A0.nmax, np);
+    const auto key = std::make_tuple(kgrad, dr, dlat, variant, nmax, np);
     auto it = c.tuned.find(key);
     if (it != c.tuned.end())
     {
         *K = it->second.first;
         return st;
     }
-    if (!autotune_on() || A0.nmax < 256 || A0.nsets > 0)
+    if (!autotune_on() || nmax < 256)
         return st;
-    std::vector<int> cands = kgrad >= 1 || dlat > 0 ? std::vector<int>{1, 2}
-                                                    : std::vector<int>{1, 2, 4};
     cudaEvent_t e0 = ev_get(c), e1 = ev_get(c);
     std::vector<std::pair<int, float>> meas;
     int best = *K;
     float best_ms = 0.0f;
-    // one untimed launch first (first-use costs of the module, caches)
-    cands.insert(cands.begin(), *K);
-    bool warm = true;
+    // every candidate runs once untimed: a kernel's first launch in a process
+    // loads its code (about 40 us, more than some of these launches take)
+    for (int k : cands)
+        CB_CUDA(launch(k), st);
     for (int k : cands)
     {
-        ShsGridArgs A = A0;
-        A.ntiles = (np + 32 * k - 1) / (32 * k);
-        A.nitems = (long long)(A.nmax + 1) * A.ntiles;
-        const int grid = (int)std::min<long long>((A.nitems + 3) / 4,
-                                                  (long long)c.num_sms * 8);
-        CB_CUDA(cudaMemsetAsync(A.counter, 0, sizeof(unsigned long long),
-                                c.stream), st);
         CB_CUDA(cudaEventRecord(e0, c.stream), st);
-        CB_CUDA(launch_shs_grid(A, kgrad, dr, dlat, rr, k, std::max(grid, 1),
-                                c.stream), st);
+        CB_CUDA(launch(k), st);
         CB_CUDA(cudaEventRecord(e1, c.stream), st);
         CB_CUDA(cudaEventSynchronize(e1), st);
         float ms = 0.0f;
         CB_CUDA(cudaEventElapsedTime(&ms, e0, e1), st);
-        c.launches++;
-        if (warm)
-        {
-            warm = false;
-            continue;
-        }
+        c.launches += 2;
         meas.emplace_back(k, ms);
         if (best_ms == 0.0f || ms < best_ms)
         {
@@ -1282,8 +1327,6 @@ Status tune_shs_k(Context &c, const ShsGridArgs &A0, int kgrad, int dr,
     }
     c.ev_pool.push_back(e0);
     c.ev_pool.push_back(e1);
-    CB_CUDA(cudaMemsetAsync(A0.counter, 0, sizeof(unsigned long long),
-                            c.stream), st);
     c.tuned[key] = std::make_pair(best, meas);
     *K = best;
     return st;
@@ -1393,6 +1436,167 @@ Status coef_to_device(Context &c, const CoefIn &in, unsigned long nmax,
     Scope sc(c, TIMER_PREP);
     CB_CUDA(launch_scale_cs((long long)nmax, (long long)in.nmax, src_c, src_s,
                             tab.tc, *dcs, c.stream), st);
+    return st;
+}
+
+// ---------------------------------------------------------------------------
+// Latitudes of a grid call on the device
+// ---------------------------------------------------------------------------
+// The latitude pairs are uploaded once and k_geometry forms what the kernels
+// read from them (and clears the call's status words).  Pairs [0, n2) run
+// the two-degree recurrence, the rest (near the equator) the one-degree one;
+// n2 = 0 keeps the whole call on the latter.
+struct GridGeo
+{
+    int np = 0, n2 = 0, polar = 0;
+    // one radius r for all rows, other than R: (R / r)^n is folded into the
+    // coefficients (rhop), the call's factor is GM / r^(dorder + 1), and rr
+    // is false
+    bool rr = false;
+    double rho = 1.0;             // R / r (1 when r = R or rr)
+    double r;                     // that r, else R
+    const double *lat, *t, *u, *z, *rhos, *w_n, *w_s;
+    const double2 *pw = nullptr;
+    const int *row_n, *row_s;
+    double *rhop = nullptr;
+    unsigned *d_status = nullptr;
+    unsigned long long *counter = nullptr;   // counter[0], counter[8]
+};
+
+// Smallest degree of the two-degree recurrence: below it a call is bound by
+// launches and by the latency of one short column, not by the FP64 pipe
+// (nmax 95: 10.7 us with it, 10.9 us without, event timings).
+constexpr unsigned long TWO_MIN_NMAX = 128;
+constexpr double TWO_NEAR = 0.05;      // |sin(lat)| (two.cuh)
+
+// Pairs that the two-degree recurrence may take: |lat| must not grow along
+// the pairs (so that neighbouring lanes are neighbouring latitudes and the
+// polar form of a 32-pair group fits all of it), from the first pair to the
+// first one within TWO_NEAR of the equator.  *polar: the leading pairs, in
+// whole groups of 32, poleward of 30 degrees.
+int two_pairs(const double *lat, int np, int *polar)
+{
+    const double near = std::asin(TWO_NEAR);
+    int n2 = np;
+    for (int p = 0; p < np; p++)
+    {
+        const double a = std::fabs(lat[p]);
+        if (p > 0 && !(a <= std::fabs(lat[p - 1])))
+            return 0;
+        if (!(a >= near) && n2 == np)
+            n2 = p;
+    }
+    // whole warps: the last up to 31 of them join the others when that leaves
+    // the others outside 0.8 TWO_NEAR
+    const int whole = (np - n2) / 32 * 32;
+    if (n2 < np && whole > 0 &&
+        std::fabs(lat[np - whole - 1]) >= std::asin(0.8 * TWO_NEAR))
+        n2 = np - whole;
+    int g = 0;
+    while (32 * (g + 1) <= n2 && std::fabs(lat[32 * g + 31]) >= PI / 6.0)
+        g++;
+    *polar = 32 * g;
+    return n2;
+}
+
+// wn, ws (analysis): the weights of the pairs' rows, or null.  r_eq: every
+// row at the coefficients' radius R (nothing to fold); allow_two: the call's
+// kernels exist in the two-degree form.
+Status grid_geometry(Context &c, const charm_point *pnt, const Pairs &P,
+                     unsigned long nmax, double R, bool r_eq, bool allow_two,
+                     double cw, bool weights, GridGeo *G)
+{
+    Status st;
+    const int np = (int)P.row_n.size();
+    G->np = np;
+    // host: lat, rho or weights (2), rows; device: the same, then t, u, z
+    const size_t up = (size_t)np * (3 * 8 + 2 * 4);
+    void *hp = nullptr;
+    CB_TRY(pinned(c, up, &hp));
+    double *hlat = static_cast<double *>(hp);
+    double *ha = hlat + np, *hb = ha + np;
+    int *hrn = reinterpret_cast<int *>(hb + np);
+    int *hrs = hrn + np;
+    bool uniform = true;
+    const double r0 = np > 0 ? pnt->r[P.row_n[0]] : R;
+    G->r = R;
+    for (int p = 0; p < np; p++)
+    {
+        const int rn = P.row_n[p], rs = P.row_s[p];
+        hlat[p] = pnt->lat[rn];
+        if (weights)
+        {
+            ha[p] = cw * pnt->w[rn];
+            hb[p] = rs >= 0 ? cw * pnt->w[rs] : 0.0;
+        }
+        else
+        {
+            ha[p] = r_eq ? 1.0 : R / pnt->r[rn];
+            uniform = uniform && pnt->r[rn] == r0;
+        }
+        hrn[p] = rn;
+        hrs[p] = rs;
+    }
+    // folding keeps every power within the range of a double with room for
+    // the chunk scaling of the one-degree tables
+    if (!weights && !r_eq)
+    {
+        const double rho = R / r0;
+        G->rr = !(uniform && std::fabs(std::log2(rho)) *
+                                     (double)(nmax + 3) <= 600.0);
+        if (!G->rr)
+        {
+            G->rho = rho;
+            G->r = r0;
+        }
+    }
+    if (allow_two && !G->rr && nmax >= TWO_MIN_NMAX)
+        G->n2 = two_pairs(hlat, np, &G->polar);
+    void *dgeo = nullptr;
+    CB_TRY(buf(c, "geo", up + (size_t)np * 3 * 8, &dgeo));
+    CB_CUDA(cudaMemcpyAsync(dgeo, hp, up, cudaMemcpyHostToDevice, c.stream),
+            st);
+    double *d = static_cast<double *>(dgeo);
+    G->lat = d;
+    G->rhos = G->w_n = d + np;
+    G->w_s = d + 2 * np;
+    G->row_n = reinterpret_cast<const int *>(d + 3 * np);
+    G->row_s = G->row_n + np;
+    double *dt = d + 4 * np;
+    G->t = dt;
+    G->u = dt + np;
+    G->z = dt + 2 * np;
+    void *sp = nullptr;
+    CB_TRY(buf(c, "status", 256, &sp));
+    G->d_status = static_cast<unsigned *>(sp);
+    G->counter = reinterpret_cast<unsigned long long *>(
+        static_cast<char *>(sp) + 64);
+    GeometryArgs A{};
+    A.npairs = np;
+    A.polar = G->polar;
+    A.lat = d;
+    A.t = dt;
+    A.u = dt + np;
+    A.z = dt + 2 * np;
+    if (G->n2 > 0)
+    {
+        double2 *pw = nullptr;
+        A.npow = 64 + (int)(nmax / 64) + 1;   // pow_entries of two.cuh
+        CB_TRY(dbuf(c, "geo_pow", (size_t)A.npow * np, &pw));
+        A.pw = pw;
+        G->pw = pw;
+    }
+    A.clear = G->d_status;
+    if (G->rho != 1.0)
+    {
+        CB_TRY(dbuf(c, "geo_rhop", (size_t)(nmax + 1), &G->rhop));
+        A.rhop = G->rhop;
+        A.nmax = (long long)nmax;
+        A.rho = G->rho;
+        A.drho = std::fma(-G->rho, r0, R) / r0 / G->rho;
+    }
+    Scope sc(c, TIMER_PREP);
+    CB_CUDA(launch_geometry(A, c.stream), st);
     return st;
 }
 
@@ -1522,51 +1726,69 @@ Status shs_grid(Context &c, const charm_point *pnt, const CoefIn &in,
     int dorder, npar;
     mur_dorder(in.mu, in.r, kgrad, dr, dlat, dlon, &mur, &dorder, &npar);
 
-    // per-pair geometry, staged through pinned memory (one upload)
-    size_t geo_bytes = (size_t)np * (3 * 8 + 2 * 4);
-    void *hp = nullptr;
-    CB_TRY(pinned(c, geo_bytes, &hp));
-    double *ht = static_cast<double *>(hp);
-    double *hu = ht + np;
-    double *hrho = hu + np;
-    int *hrn = reinterpret_cast<int *>(hrho + np);
-    int *hrs = hrn + np;
-    for (int p = 0; p < np; p++)
-    {
-        double la = pnt->lat[P.row_n[p]];
-        sincos(la, &ht[p], &hu[p]);
-        hrho[p] = r_eq ? 1.0 : in.r / pnt->r[P.row_n[p]];
-        hrn[p] = P.row_n[p];
-        hrs[p] = P.row_s[p];
-    }
-    void *dgeo = nullptr;
-    CB_TRY(buf(c, "geo", geo_bytes, &dgeo));
-    CB_CUDA(cudaMemcpyAsync(dgeo, hp, geo_bytes, cudaMemcpyHostToDevice,
-                            c.stream), st);
-    const double *dt = static_cast<const double *>(dgeo);
-    const double *du = dt + np;
-    const double *drho = du + np;
-    const int *drn = reinterpret_cast<const int *>(drho + np);
-    const int *drs = drn + np;
+    // the two-degree recurrence serves the quantities without a latitudinal
+    // derivative
+    GridGeo G;
+    CB_TRY(grid_geometry(c, pnt, P, nmax, in.r, r_eq,
+                         kgrad == 0 && dlat == 0, 0.0, false, &G));
+    mur_dorder(in.mu, G.r, kgrad, dr, dlat, dlon, &mur, &dorder, &npar);
+    const int n2 = G.n2;
 
     Tabs tab;
-    CB_TRY(tables(c, (long long)nmax, &tab));
+    CB_TRY(tables(c, (long long)nmax, &tab, n2 > 0));
+    const bool old_too = n2 < np;   // some latitudes on the one-degree path
     // Host coefficients of a call whose grid goes to the host are uploaded
     // later, in bands of orders overlapped with the synthesis of the first
     // band of latitudes (when the call runs in bands), else all now.
-    double2 *dcs = nullptr;
+    double2 *dcs = nullptr, *dcs2 = nullptr;
+    const double *src_c = in.dc, *src_s = in.ds;
     double *raw = nullptr;
     const long long Ts = (long long)(in.nmax + 1) * (in.nmax + 2) / 2;
+    const int variant = (G.rr ? 1 : 0) + (n2 > 0 ? 2 : 0);
     bool coef_later =
         !in.dc && !d_f &&
-        shs_k_settled(c, kgrad, dr, dlat, !r_eq, (long long)nmax, np);
-    if (coef_later)
-    {
+        shs_k_settled(c, kgrad, dr, dlat, variant, (long long)nmax, np);
+    if (old_too)
         CB_TRY(dbuf(c, "cs", (size_t)((nmax + 1) * (nmax + 2) / 2), &dcs));
+    if (n2 > 0)
+        CB_TRY(dbuf(c, "cs2", (size_t)(2 * two_steps((long long)nmax)),
+                    &dcs2));
+    if (!in.dc)
+    {
         CB_TRY(dbuf(c, "shc_in", (size_t)(2 * Ts), &raw));
+        src_c = raw;
+        src_s = raw + Ts;
     }
-    else
-        CB_TRY(coef_to_device(c, in, nmax, tab, &dcs));
+    // the kernels' form of the coefficients of the orders [m_lo, m_hi)
+    auto scale = [&](long long m_lo, long long m_hi) -> Status {
+        Status s2;
+        Scope sc(c, TIMER_PREP);
+        ScaleArgs S{};
+        S.ntab = S.nmax = (long long)nmax;
+        S.shc_nmax = (long long)in.nmax;
+        S.c = src_c;
+        S.s = src_s;
+        S.tc = tab.tc;
+        S.kw = tab.kw;
+        S.rhop = G.rhop;
+        S.dr = dr;
+        S.cs = dcs;
+        S.cs2 = dcs2;
+        CB_CUDA(launch_scale_orders(S, m_lo, m_hi, c.stream), s2);
+        return s2;
+    };
+    auto all_coefs = [&]() -> Status {
+        Status s2;
+        if (!in.dc)
+        {
+            CB_TRY(upload_tri(c, in.hc, in.nmax, raw));
+            CB_TRY(upload_tri(c, in.hs, in.nmax, raw + Ts));
+        }
+        CB_TRY(scale(0, (long long)nmax + 1));
+        return s2;
+    };
+    if (!coef_later)
+        CB_TRY(all_coefs());
 
     // lumped coefficients
     const int ldf = use_fft ? (int)(nlon / 2 + 1) : (int)(nmax + 1);
@@ -1591,27 +1813,21 @@ Status shs_grid(Context &c, const charm_point *pnt, const CoefIn &in,
         CB_TRY(row_fft(c, (long long)nlon, &rf));
         CB_TRY(row_fft_quarter(c, (long long)nlon, rf, &rfq));
     }
-    unsigned *d_status;
-    unsigned long long *d_counter;
-    CB_TRY(status_words(c, &d_status, &d_counter));
+    unsigned *const d_status = G.d_status;
 
-    int K = choose_k(kgrad, dlat, np);
-    int ntiles = (np + 32 * K - 1) / (32 * K);
     ShsGridArgs A{};
     A.nmax = (long long)nmax;
-    A.npairs = np;
-    A.ntiles = ntiles;
-    A.nitems = (long long)(nmax + 1) * ntiles;
     A.tb = tab.tb;
     A.tmul = tab.tmul;
     A.ldmul = tab.ldmul;
     A.sg = tab.sg;
+    A.npairs = np;
     A.cs = dcs;
-    A.t = dt;
-    A.u = du;
-    A.rho = drho;
-    A.row_n = drn;
-    A.row_s = drs;
+    A.t = G.t;
+    A.u = G.u;
+    A.rho = G.rhos;
+    A.row_n = G.row_n;
+    A.row_s = G.row_s;
     A.nlat = (int)nlat;
     A.ldf = ldf;
     A.out = lc;
@@ -1619,25 +1835,99 @@ Status shs_grid(Context &c, const charm_point *pnt, const CoefIn &in,
     A.fft_pack = use_fft ? 1 : 0;
     A.dlon = dlon;
     A.polar_thr = polar_threshold(nmax);
-    A.counter = d_counter;
     A.status = d_status;
+    ShsTwoArgs B{};
+    B.nmax = (long long)nmax;
+    B.npairs = n2;
+    B.polar = G.polar;
+    B.ab = tab.ab;
+    B.ag = tab.ag;
+    B.sm = tab.sm;
+    B.sg = tab.sg;
+    B.cs = dcs2;
+    B.t = G.t;
+    B.u = G.u;
+    B.z = G.z;
+    B.pw = G.pw;
+    B.pw_ld = np;
+    B.tb = tab.tb;
+    B.tmul = tab.tmul;
+    B.ldmul = tab.ldmul;
+    B.cs1 = dcs;
+    B.row_n = G.row_n;
+    B.row_s = G.row_s;
+    B.nlat = (int)nlat;
+    B.ldf = ldf;
+    B.out = lc;
+    B.mur = mur;
+    B.fft_pack = A.fft_pack;
+    B.dr = dr;
+    B.dlon = dlon;
+    B.polar_thr = A.polar_thr;
+    B.status = d_status;
+    auto blocks = [&](long long items) {
+        return (int)std::max<long long>(
+            1, std::min<long long>((items + 3) / 4, (long long)c.num_sms * 8));
+    };
+    // synthesis of the orders [m_lo, m_hi) and the pairs [p0, p1) (p0 a
+    // multiple of 32 K): the two-degree kernel, which takes the pairs from
+    // n2 on through the one-degree recurrence itself, or the one-degree
+    // kernel for the whole call; cnt: a cleared counter
+    auto synth = [&](int K, int p0, int p1, long long m_lo, long long m_hi,
+                     unsigned long long *cnt) {
+        if (n2 > 0)
+        {
+            ShsTwoArgs b = B;
+            const int q = std::min(p1, n2);
+            b.tile0 = p0 / (32 * K);
+            b.ntiles = p0 < q ? (q - p0 + 32 * K - 1) / (32 * K) : 0;
+            b.near0 = std::max(p0, n2);
+            b.nnear = std::max(0, p1 - b.near0);
+            b.near_tiles = (b.nnear + SHS_NEAR_PAIRS - 1) / SHS_NEAR_PAIRS;
+            b.m0 = m_lo;
+            b.nitems = (m_hi - m_lo) * (b.ntiles + b.near_tiles);
+            b.counter = cnt;
+            return launch_shs_two(b, K, blocks(b.nitems), c.stream);
+        }
+        ShsGridArgs a = A;
+        a.tile0 = p0 / (32 * K);
+        a.ntiles = (p1 - p0 + 32 * K - 1) / (32 * K);
+        a.m0 = m_lo;
+        a.nitems = (m_hi - m_lo) * a.ntiles;
+        a.counter = cnt;
+        return launch_shs_grid(a, kgrad, dr, dlat, G.rr, K, blocks(a.nitems),
+                               c.stream);
+    };
+    int K = n2 > 0 ? choose_k_two(n2) : choose_k(kgrad, dlat, np);
     // autotuned tile (first call of this shape)
     {
-        int Kt = K;
-        CB_TRY(tune_shs_k(c, A, kgrad, dr, dlat, !r_eq, np, &Kt));
-        if (Kt != K)
-        {
-            K = Kt;
-            ntiles = (np + 32 * K - 1) / (32 * K);
-            A.ntiles = ntiles;
-            A.nitems = (long long)(nmax + 1) * ntiles;
-        }
+        auto trial = [&](int k) {
+            const cudaError_t e = cudaMemsetAsync(
+                G.counter, 0, sizeof(unsigned long long), c.stream);
+            return e != cudaSuccess ? e
+                                    : synth(k, 0, np, 0, (long long)nmax + 1,
+                                            G.counter);
+        };
+        const bool timed = !shs_k_settled(c, kgrad, dr, dlat, variant,
+                                          (long long)nmax, np);
+        std::vector<int> cands =
+            kgrad >= 1 || dlat > 0 ? std::vector<int>{1, 2}
+                                   : std::vector<int>{1, 2, 4};
+        if (n2 > 0)
+            cands = n2 <= 1024 ? std::vector<int>{1, 2, 3, 4, 5, 6}
+                               : std::vector<int>{3, 4, 5, 6, 7, 8};
+        CB_TRY(tune_shs_k(c, trial, cands, kgrad, dr, dlat, variant,
+                          (long long)nmax, np, &K));
+        if (timed)
+            CB_CUDA(cudaMemsetAsync(G.counter, 0, sizeof(unsigned long long),
+                                    c.stream), st);
     }
 
     // Host output through the row transform: bands of latitude tiles, each
     // band's rows copied to the host (copy stream) while the next band is
     // synthesised; the sums of every item are the same as in one launch.
     std::vector<std::array<int, 6>> bands;
+    const int ntiles = (np + 32 * K - 1) / (32 * K);
     const int nband =
         (!d_f && rf) ? grid_bands(P, (int)nlat, ntiles, 32 * K,
                                   ntiles >= 6 ? SHS_LAT_BANDS : 2, bands)
@@ -1645,12 +1935,7 @@ Status shs_grid(Context &c, const charm_point *pnt, const CoefIn &in,
     if (coef_later && nband <= 1)
     {
         // no bands: every coefficient now
-        CB_TRY(upload_tri(c, in.hc, in.nmax, raw));
-        CB_TRY(upload_tri(c, in.hs, in.nmax, raw + Ts));
-        Scope sc(c, TIMER_PREP);
-        CB_CUDA(launch_scale_cs((long long)nmax, (long long)in.nmax, raw,
-                                raw + Ts, tab.tc, dcs, c.stream),
-                st);
+        CB_TRY(all_coefs());
         coef_later = false;
     }
     if (nband > 1)
@@ -1694,6 +1979,8 @@ Status shs_grid(Context &c, const charm_point *pnt, const CoefIn &in,
         for (int b = 0; b < nband; b++)
         {
             const auto &bd = bands[b];
+            const int p0 = std::min(np, bd[0] * 32 * K);
+            const int p1 = std::min(np, bd[1] * 32 * K);
             // the first band synthesises each band of orders as soon as its
             // coefficients are on the device
             const bool split = b == 0 && coef_later;
@@ -1704,26 +1991,12 @@ Status shs_grid(Context &c, const charm_point *pnt, const CoefIn &in,
                     CB_CUDA(cudaStreamWaitEvent(c.stream, c.band_ev[EV_ORD0 + k],
                                                 0),
                             st);
-                    Scope sc(c, TIMER_PREP);
-                    CB_CUDA(launch_scale_cs_orders(
-                                (long long)nmax, (long long)in.nmax, raw,
-                                raw + Ts, tab.tc, dcs, mb[k], mb[k + 1],
-                                c.stream),
-                            st);
+                    CB_TRY(scale(mb[k], mb[k + 1]));
                 }
-                ShsGridArgs Ab = A;
-                Ab.tile0 = bd[0];
-                Ab.ntiles = bd[1] - bd[0];
-                Ab.m0 = split ? mb[k] : 0;
-                Ab.nitems = (long long)(split ? mb[k + 1] - mb[k]
-                                              : (long long)nmax + 1) *
-                            Ab.ntiles;
-                Ab.counter = bcnt + (split ? 8 + k : b);
-                const int gb = (int)std::min<long long>(
-                    (Ab.nitems + 3) / 4, (long long)c.num_sms * 8);
                 Scope sc(c, TIMER_SHS);
-                CB_CUDA(launch_shs_grid(Ab, kgrad, dr, dlat, !r_eq, K,
-                                        std::max(gb, 1), c.stream), st);
+                CB_CUDA(synth(K, p0, p1, split ? mb[k] : 0,
+                              split ? mb[k + 1] : (long long)nmax + 1,
+                              bcnt + (split ? 8 + k : b)), st);
             }
             for (int q = 0; q < npar; q++)
                 for (int h = 0; h < 2; h++)
@@ -1762,12 +2035,9 @@ Status shs_grid(Context &c, const charm_point *pnt, const CoefIn &in,
         return finish(c, d_status);
     }
 
-    int grid = (int)std::min<long long>((A.nitems + 3) / 4,
-                                        (long long)c.num_sms * 8);
     {
         Scope sc(c, TIMER_SHS);
-        CB_CUDA(launch_shs_grid(A, kgrad, dr, dlat, !r_eq, K,
-                                std::max(grid, 1), c.stream), st);
+        CB_CUDA(synth(K, 0, np, 0, (long long)nmax + 1, G.counter), st);
     }
 
     // longitude sums into the output grid(s)
@@ -1887,10 +2157,12 @@ struct BatchGeo
     const double *dt = nullptr;   // t[np], u[np], rho[np], row_n, row_s
 };
 
-Status batch_geometry(Context &c, const charm_point *pnt, unsigned long N,
-                      double R, BatchGeo *G)
+// checks and pairs only
+Status batch_pairs(Context &c, const charm_point *pnt, unsigned long N,
+                   double R, BatchGeo *G)
 {
     Status st;
+    (void)c;
     const double thr = charm_glob_threshold, thr2 = charm_glob_threshold2;
     const size_t nlat = pnt->nlat, nlon = pnt->nlon;
     if (pnt->type == CHARM_CRD_POINT_GRID && nlon > 1)
@@ -1929,7 +2201,19 @@ Status batch_geometry(Context &c, const charm_point *pnt, unsigned long N,
                 grid_pairs(pnt, thr2, false, P);
                 break;
             }
-    const int np = (int)P.row_n.size();
+    G->np = (int)P.row_n.size();
+    G->r_eq = r_eq;
+    return st;
+}
+
+Status batch_geometry(Context &c, const charm_point *pnt, unsigned long N,
+                      double R, BatchGeo *G)
+{
+    Status st;
+    CB_TRY(batch_pairs(c, pnt, N, R, G));
+    const Pairs &P = G->P;
+    const bool r_eq = G->r_eq;
+    const int np = G->np;
     size_t geo_bytes = (size_t)np * (3 * 8 + 2 * 4);
     void *hp = nullptr;
     CB_TRY(pinned(c, geo_bytes, &hp));
@@ -1950,11 +2234,7 @@ Status batch_geometry(Context &c, const charm_point *pnt, unsigned long N,
     CB_TRY(buf(c, "geo", geo_bytes, &dgeo));
     CB_CUDA(cudaMemcpyAsync(dgeo, hp, geo_bytes, cudaMemcpyHostToDevice,
                             c.stream), st);
-    const double *dt = static_cast<const double *>(dgeo);
-
-    G->np = np;
-    G->r_eq = r_eq;
-    G->dt = dt;
+    G->dt = static_cast<const double *>(dgeo);
     return st;
 }
 
@@ -1972,42 +2252,51 @@ Status shs_batch(Context &c, const charm_point *pnt, size_t nsets,
                  const double *const *d_s, int kgrad, double *const *d_f)
 {
     Status st;
-    const double thr = charm_glob_threshold, thr2 = charm_glob_threshold2;
     const size_t nlat = pnt->nlat, nlon = pnt->nlon;
     unsigned long N = 0;
     for (size_t j = 0; j < nsets; j++)
         N = std::max(N, nmax_v[j]);
-    BatchGeo G;
-    CB_TRY(batch_geometry(c, pnt, N, R, &G));
-    const Pairs &P = G.P;
-    const int np = G.np;
-    const bool r_eq = G.r_eq;
-    const double *dt = G.dt;
-    (void)thr;
-    (void)thr2;
-    (void)P;
+    BatchGeo BG;
+    CB_TRY(batch_pairs(c, pnt, N, R, &BG));
+    const int np = BG.np;
+    GridGeo G;
+    CB_TRY(grid_geometry(c, pnt, BG.P, N, R, BG.r_eq,
+                         kgrad == 0 || kgrad == 3, 0.0, false, &G));
+    const int n2 = G.n2;
+    // the gradient kinds stay with the one-degree recurrence
+    const bool old_too = n2 < np || kgrad != 0;
 
     Tabs tab;
-    CB_TRY(tables(c, (long long)N, &tab));
+    CB_TRY(tables(c, (long long)N, &tab, n2 > 0));
     const long long T = (long long)(N + 1) * (N + 2) / 2;
-    double2 *cs_all = nullptr;
-    CB_TRY(dbuf(c, "batch_cs", (size_t)nsets * T, &cs_all));
+    const long long T2 = 2 * two_steps((long long)N);
+    double2 *cs_all = nullptr, *cs2_all = nullptr;
+    if (old_too)
+        CB_TRY(dbuf(c, "batch_cs", (size_t)nsets * T, &cs_all));
+    if (n2 > 0)
+        CB_TRY(dbuf(c, "batch_cs2", (size_t)nsets * T2, &cs2_all));
     for (size_t j = 0; j < nsets; j++)
     {
+        ScaleArgs S{};
+        S.ntab = (long long)N;
+        S.nmax = (long long)nmax_v[j];
+        S.shc_nmax = (long long)shc_nmax_v[j];
+        S.c = d_c[j];
+        S.s = d_s[j];
+        S.tc = tab.tc;
+        S.kw = tab.kw;
+        S.rhop = G.rhop;
+        S.cs = cs_all ? cs_all + (size_t)j * T : nullptr;
+        S.cs2 = cs2_all ? cs2_all + (size_t)j * T2 : nullptr;
         Scope sc(c, TIMER_PREP);
-        CB_CUDA(launch_scale_cs_set((long long)N, (long long)nmax_v[j],
-                                    (long long)shc_nmax_v[j], d_c[j], d_s[j],
-                                    tab.tc, cs_all + (size_t)j * T, c.stream),
-                st);
+        CB_CUDA(launch_scale_orders(S, 0, S.nmax + 1, c.stream), st);
     }
     const RfftArgs *rf = nullptr, *rfq = nullptr;
     CB_TRY(row_fft(c, (long long)nlon, &rf));
     CB_TRY(row_fft_quarter(c, (long long)nlon, rf, &rfq));
     const int ldf = (int)(nlon / 2 + 1);
     const size_t grid_sz = nlat * nlon;
-    unsigned *d_status;
-    unsigned long long *d_counter;
-    CB_TRY(status_words(c, &d_status, &d_counter));
+    unsigned *const d_status = G.d_status;
 
     // derivative kinds of this call and where their components go in the
     // caller's per-set output (CHarm's order after its pointer reordering,
@@ -2047,8 +2336,11 @@ Status shs_batch(Context &c, const charm_point *pnt, size_t nsets,
         BatchSet *dsets = nullptr;
         CB_TRY(dbuf(c, "batch_sets", bsz, &dsets));
         std::vector<BatchSet> hsets(bsz);
-        const int K = choose_k(kg, dd, np);
-        const int ntiles = (np + 32 * K - 1) / (32 * K);
+        const bool two = kg == 0 && n2 > 0;
+        const int K = two ? choose_k_two(n2) : choose_k(kg, dd, np);
+        const int near = two ? (np - n2 + SHS_NEAR_PAIRS - 1) / SHS_NEAR_PAIRS
+                             : 0;
+        const int ntiles = ((two ? n2 : np) + 32 * K - 1) / (32 * K);
         for (size_t j0 = 0; j0 < nsets; j0 += bsz)
         {
             const size_t nb = std::min(bsz, nsets - j0);
@@ -2058,47 +2350,85 @@ Status shs_batch(Context &c, const charm_point *pnt, size_t nsets,
                 const size_t j = j0 + b;
                 double mur;
                 int dorder, npar_j;
-                mur_dorder(mu_v[j], R, kg, dd, dd, dd, &mur, &dorder,
+                mur_dorder(mu_v[j], G.r, kg, dd, dd, dd, &mur, &dorder,
                            &npar_j);
                 hsets[b].nmax = (long long)nmax_v[j];
                 hsets[b].item0 = items;
-                hsets[b].cs = cs_all + j * T;
+                hsets[b].cs1 = cs_all ? cs_all + j * T : nullptr;
+                hsets[b].cs = two ? cs2_all + j * T2 : hsets[b].cs1;
                 hsets[b].out = lc + b * (per_set / sizeof(double2));
                 hsets[b].mur = mur;
                 hsets[b].polar_thr = polar_threshold(nmax_v[j]);
-                items += (long long)(nmax_v[j] + 1) * ntiles;
+                items += (long long)(nmax_v[j] + 1) * (ntiles + near);
             }
             CB_TRY(h2d_small(c, dsets, hsets.data(), nb * sizeof(BatchSet)));
-            CB_CUDA(cudaMemsetAsync(d_counter, 0, sizeof(unsigned long long),
+            CB_CUDA(cudaMemsetAsync(G.counter, 0, sizeof(unsigned long long),
                                     c.stream), st);
-            ShsGridArgs A{};
-            A.nmax = (long long)N;
-            A.npairs = np;
-            A.ntiles = ntiles;
-            A.nitems = items;
-            A.tb = tab.tb;
-            A.tmul = tab.tmul;
-            A.ldmul = tab.ldmul;
-            A.sg = tab.sg;
-            A.t = dt;
-            A.u = dt + np;
-            A.rho = dt + 2 * np;
-            A.row_n = reinterpret_cast<const int *>(dt + 3 * np);
-            A.row_s = A.row_n + np;
-            A.nlat = (int)nlat;
-            A.ldf = ldf;
-            A.fft_pack = 1;
-            A.dlon = dd;
-            A.counter = d_counter;
-            A.status = d_status;
-            A.sets = dsets;
-            A.nsets = (int)nb;
-            int grid = (int)std::min<long long>((items + 3) / 4,
-                                                (long long)c.num_sms * 8);
+            const int grid = (int)std::max<long long>(
+                1, std::min<long long>((items + 3) / 4,
+                                       (long long)c.num_sms * 8));
+            if (two)
             {
+                ShsTwoArgs B{};
+                B.nmax = (long long)N;
+                B.npairs = n2;
+                B.polar = G.polar;
+                B.ntiles = ntiles;
+                B.near0 = n2;
+                B.nnear = np - n2;
+                B.near_tiles = near;
+                B.nitems = items;
+                B.ab = tab.ab;
+                B.ag = tab.ag;
+                B.sm = tab.sm;
+                B.sg = tab.sg;
+                B.t = G.t;
+                B.u = G.u;
+                B.z = G.z;
+                B.pw = G.pw;
+                B.pw_ld = np;
+                B.tb = tab.tb;
+                B.tmul = tab.tmul;
+                B.ldmul = tab.ldmul;
+                B.row_n = G.row_n;
+                B.row_s = G.row_s;
+                B.nlat = (int)nlat;
+                B.ldf = ldf;
+                B.fft_pack = 1;
+                B.counter = G.counter;
+                B.status = d_status;
+                B.sets = dsets;
+                B.nsets = (int)nb;
                 Scope sc(c, TIMER_SHS);
-                CB_CUDA(launch_shs_grid(A, kg, dd, dd, !r_eq, K,
-                                        std::max(grid, 1), c.stream), st);
+                CB_CUDA(launch_shs_two(B, K, grid, c.stream), st);
+            }
+            else
+            {
+                ShsGridArgs A{};
+                A.nmax = (long long)N;
+                A.npairs = np;
+                A.ntiles = ntiles;
+                A.nitems = items;
+                A.tb = tab.tb;
+                A.tmul = tab.tmul;
+                A.ldmul = tab.ldmul;
+                A.sg = tab.sg;
+                A.t = G.t;
+                A.u = G.u;
+                A.rho = G.rhos;
+                A.row_n = G.row_n;
+                A.row_s = G.row_s;
+                A.nlat = (int)nlat;
+                A.ldf = ldf;
+                A.fft_pack = 1;
+                A.dlon = dd;
+                A.counter = G.counter;
+                A.status = d_status;
+                A.sets = dsets;
+                A.nsets = (int)nb;
+                Scope sc(c, TIMER_SHS);
+                CB_CUDA(launch_shs_grid(A, kg, dd, dd, G.rr, K, grid,
+                                        c.stream), st);
             }
             // longitude transforms, component by component into the
             // caller's output slots

@@ -25,6 +25,7 @@ struct BatchSet
     long long nmax;
     long long item0;
     const double2 *cs;
+    const double2 *cs1;   // one-degree form beside a two-degree cs
     double2 *out;
     double mur;
     double polar_thr;
@@ -65,6 +66,79 @@ struct ShsGridArgs
     // nmax), cs, out, mur and polar_thr replace the fields above
     const BatchSet *sets;
     int nsets;
+};
+
+// Grid synthesis of the potential and its radial derivatives with the
+// two-degree recurrence (shs_two.cu, two.cuh); fields as ShsGridArgs.
+struct ShsTwoArgs
+{
+    long long nmax;
+    int npairs;            // pairs [0, npairs) of the geometry arrays
+    int polar;             // pairs below this take z = -cos^2 (multiple of 32)
+    int ntiles;
+    int tile0;
+    long long m0;
+    long long nitems;      // orders x (near_tiles + ntiles), all sets
+    const double2 *ab, *ag;   // (alpha, beta), (alpha, gamma) per step
+    const double *sm;      // S_m per order
+    const double *sg;
+    const double2 *cs;     // coefficient pairs of k_two_scale
+    const double *t, *u, *z;
+    const double2 *pw;     // powers of u (two_seed), row length pw_ld
+    int pw_ld;
+    // pairs [near0, near0 + nnear) of the geometry arrays run the one-degree
+    // recurrence, in near_tiles tiles that come first among the items
+    int near0, nnear, near_tiles;
+    const double2 *tb;     // one-degree tables and coefficients (leg.cuh)
+    const double *tmul;
+    int ldmul;
+    const double2 *cs1;
+    const int *row_n, *row_s;
+    int nlat;
+    int ldf;
+    double2 *out;
+    double mur;
+    int fft_pack;
+    int dr, dlon;          // radial and longitudinal derivative orders
+    double polar_thr;
+    unsigned long long *counter;
+    unsigned *status;
+    const BatchSet *sets;  // cs (two-degree) and cs1 per set
+    int nsets;
+};
+
+// Latitudes of the evaluated pairs on the device (two_tables.cu).
+constexpr int GEO_CLEAR_WORDS = 64;
+struct GeometryArgs
+{
+    int npairs;
+    int polar;             // pairs below this store z = -cos^2, else sin^2
+    const double *lat;
+    double *t, *u, *z;
+    double2 *pw;           // power table of two_seed, npow entries (or 0)
+    int npow;
+    unsigned *clear;       // GEO_CLEAR_WORDS words to zero
+    // powers rho^n of one radius ratio, or rhop null
+    double *rhop;
+    long long nmax;
+    double rho, drho;
+};
+
+// Coefficients of one set into the forms the grid syntheses read
+// (k_two_scale, k_scale_cs).
+struct ScaleArgs
+{
+    long long ntab;          // degree of the tables (layout of cs, cs2)
+    long long nmax;          // degree of the set
+    long long shc_nmax;      // degree of the triangles c, s
+    const double *c, *s;
+    const double *tc;        // ct_n of the one-degree tables
+    const double *kw;        // weights of k_two_tables
+    const double *rhop;      // factor of degree n, or null
+    int dr;                  // radial derivative order folded into cs2 (and
+                             // into cs beside it)
+    double2 *cs;             // one-degree form, or null
+    double2 *cs2;            // two-degree form, or null
 };
 
 // Grid analysis: C_nm, S_nm partial sums per latitude group (sha_grid.cu).
@@ -271,19 +345,13 @@ cudaError_t launch_tables(long long nmax, const double *r, const double *ri,
                           double *tmul, int ldmul, double *sg,
                           cudaStream_t st);
 // k_scale_cs for the orders [m_lo, m_hi) only
-cudaError_t launch_scale_cs_orders(long long nmax, long long shc_nmax,
-                                   const double *c, const double *s,
-                                   const double *tc, double2 *cs,
-                                   long long m_lo, long long m_hi,
-                                   cudaStream_t st);
+// orders [m_lo, m_hi) in the forms A asks for
+cudaError_t launch_scale_orders(const ScaleArgs &A, long long m_lo,
+                                long long m_hi, cudaStream_t st);
 cudaError_t launch_scale_cs(long long nmax, long long shc_nmax,
                             const double *c, const double *s,
                             const double *tc, double2 *cs, cudaStream_t st);
 // same into the layout of degree ntab >= nmax (zero above nmax)
-cudaError_t launch_scale_cs_set(long long ntab, long long nmax,
-                                long long shc_nmax, const double *c,
-                                const double *s, const double *tc,
-                                double2 *cs, cudaStream_t st);
 cudaError_t launch_shs_grid(const ShsGridArgs &A, int kgrad, int dr,
                             int dlat, bool rr, int K, int grid,
                             cudaStream_t st);
@@ -308,6 +376,18 @@ cudaError_t launch_sha_reduce(long long nmax, long long shc_nmax, int ngroups,
                               const double *tc, const double *rescale,
                               double scale, double *c, double *s,
                               cudaStream_t st);
+// sg: the finished one-degree seeds factors; sm[m] receives S_m
+cudaError_t launch_two_tables(long long nmax, const double *sg, double2 *ab,
+                              double2 *ag, double *kw, double *sm,
+                              cudaStream_t st);
+cudaError_t launch_geometry(const GeometryArgs &G, cudaStream_t st);
+// orders [m_lo, m_hi); A.cs2 must not be null
+cudaError_t launch_two_scale(const ScaleArgs &A, long long m_lo,
+                             long long m_hi, cudaStream_t st);
+// K latitude pairs per lane, 1..8; near tiles hold SHS_NEAR_PAIRS pairs
+constexpr int SHS_NEAR_PAIRS = 32;
+cudaError_t launch_shs_two(const ShsTwoArgs &A, int K, int grid,
+                           cudaStream_t st);
 cudaError_t launch_gl_nodes(unsigned long nmax, double *lat, double *w,
                             unsigned *status, cudaStream_t st);
 cudaError_t launch_dh_nodes(unsigned long nmax, double *lat, double *w,

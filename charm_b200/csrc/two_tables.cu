@@ -1,0 +1,355 @@
+// Tables of the two-degree recurrence (two.cuh), the latitudes of a grid in
+// the form its kernels read, and the passes that take coefficients into and
+// out of its normalisation.
+#include <cstdint>
+
+#include "common.cuh"
+#include "kernels.h"
+#include "two.cuh"
+
+namespace cb
+{
+
+namespace
+{
+
+// eps_n^2 of order m at n = m + i, in double-double (the products are exact
+// integers below 2^53)
+__device__ __forceinline__ dd eps2(long long m, long long i)
+{
+    const double num = (double)i * (double)(2 * m + i);
+    const double n = (double)(m + i);
+    return dd_div(dd{num, 0.0}, dd{4.0 * n * n - 1.0, 0.0});
+}
+
+// k_l+1^2 / k_l-1^2
+__device__ __forceinline__ dd k_ratio(long long m, long long l)
+{
+    const double i = 2.0 * (double)l, d = (double)(2 * m), n = i + (double)m;
+    // (eps_i+1 eps_i)^2 / (eps_i+2 eps_i+3)^2, each factor exact
+    dd num = dd_mul(dd{(i + 1.0) * (d + i + 1.0), 0.0}, dd{i * (d + i), 0.0});
+    num = dd_mul(num, dd_mul(dd{4.0 * (n + 2.0) * (n + 2.0) - 1.0, 0.0},
+                             dd{4.0 * (n + 3.0) * (n + 3.0) - 1.0, 0.0}));
+    dd den = dd_mul(dd{(i + 2.0) * (d + i + 2.0), 0.0},
+                    dd{(i + 3.0) * (d + i + 3.0), 0.0});
+    den = dd_mul(den, dd_mul(dd{4.0 * n * n - 1.0, 0.0},
+                             dd{4.0 * (n + 1.0) * (n + 1.0) - 1.0, 0.0}));
+    return dd_div(num, den);
+}
+
+constexpr int TAB_THREADS = 128;
+
+} // namespace
+
+// One block per order.  k_l^2 is a product of k_ratio over every second l
+// (two interleaved chains from k_0, k_1): each thread multiplies a
+// contiguous stretch of l, the block scans the stretches, and the second
+// walk writes
+//     ab = (alpha_l, beta_l),  ag = (alpha_l, gamma_l),
+//     kw = (k_l eps_m+2l+1, k_l eps_m+2l+2, k_l),
+// and sm[m] = S_m = P_mm / cos^m.
+// k_0 = 1 / eps_m+1, so s_0 = P_mm; k_1 = k_0 sqrt(k_ratio(1)) rounded (any
+// value serves; this one keeps the two chains level).
+__global__ void k_two_tables(long long nmax, const double *sg, double2 *ab,
+                             double2 *ag, double *kw, double *sm, long long TL)
+{
+    if (threadIdx.x == 0)
+        sm[blockIdx.x] = scalbn(sg[2 * blockIdx.x],
+                                -(int)sg[2 * blockIdx.x + 1]);
+    __shared__ dd chain[2][TAB_THREADS];
+    const long long m = blockIdx.x;
+    const long long nl = two_len(nmax, m);
+    const long long c0 = two_col0(nmax, m);
+    const int tid = threadIdx.x;
+    // even stretches keep the parity of l fixed per slot
+    const long long len = 2 * ((nl + 1 + 2 * TAB_THREADS - 1) /
+                               (2 * TAB_THREADS));
+    const long long l0 = tid * len;
+    // k^2 of l0 and l0 + 1 relative to k^2 of 0 and 1: the products over the
+    // stretches before this one
+    dd p0{1.0, 0.0}, p1{1.0, 0.0};
+    for (long long l = l0; l < l0 + len && l <= nl; l += 2)
+    {
+        p0 = dd_mul(p0, k_ratio(m, l + 1));   // k_l+2 / k_l
+        p1 = dd_mul(p1, k_ratio(m, l + 2));   // k_l+3 / k_l+1
+    }
+    chain[0][tid] = p0;
+    chain[1][tid] = p1;
+    __syncthreads();
+    for (int off = 1; off < TAB_THREADS; off <<= 1)
+    {
+        dd a0{1.0, 0.0}, a1{1.0, 0.0};
+        if (tid >= off)
+        {
+            a0 = chain[0][tid - off];
+            a1 = chain[1][tid - off];
+        }
+        __syncthreads();
+        if (tid >= off)
+        {
+            chain[0][tid] = dd_mul(a0, chain[0][tid]);
+            chain[1][tid] = dd_mul(a1, chain[1][tid]);
+        }
+        __syncthreads();
+    }
+    const dd k0sq = dd_div(dd{1.0, 0.0}, eps2(m, 1));
+    const double r1 = sqrt(k_ratio(m, 1).hi);
+    dd ke = k0sq, ko = dd_mul(k0sq, dd{r1, 0.0});
+    if (tid > 0)
+    {
+        ke = dd_mul(ke, chain[0][tid - 1]);
+        ko = dd_mul(ko, chain[1][tid - 1]);
+    }
+    for (long long l = l0; l < l0 + len && l < nl; l += 2)
+    {
+        // k_l^2 = ke, k_l+1^2 = ko, k_l+2^2
+        const dd kn = dd_mul(ke, k_ratio(m, l + 1));
+        dd ks[3] = {ke, ko, kn};
+#pragma unroll
+        for (int h = 0; h < 2; h++)
+        {
+            const long long ll = l + h;
+            if (ll >= nl)
+                break;
+            const dd e1 = eps2(m, 2 * ll + 1), e2 = eps2(m, 2 * ll + 2),
+                     e3 = eps2(m, 2 * ll + 3);
+            const dd alpha = dd_sqrt(
+                dd_div(ks[h], dd_mul(ks[h + 1], dd_mul(e2, e3))));
+            const dd A = dd_add(e1, e2);
+            const dd beta = dd_neg(dd_mul(A, alpha));
+            const dd gamma = dd_add(alpha, beta);
+            ab[c0 + ll] = make_double2(alpha.hi, beta.hi);
+            ag[c0 + ll] = make_double2(alpha.hi, gamma.hi);
+            kw[c0 + ll] = dd_sqrt(dd_mul(ks[h], e1)).hi;
+            kw[TL + c0 + ll] = dd_sqrt(dd_mul(ks[h], e2)).hi;
+            kw[2 * TL + c0 + ll] = dd_sqrt(ks[h]).hi;
+        }
+        const dd kon = dd_mul(ko, k_ratio(m, l + 2));
+        ke = kn;
+        ko = kon;
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Latitudes.  Per pair, from the double-double sine and cosine of its
+// latitude (Taylor series of lat / 8, doubled three times): t, u rounded;
+// z = x2, or -u2 for the pairs below `polar`; and (blockIdx.y > 0) the power
+// table of two_seed, POW_STRETCH entries per thread.  The first block also
+// clears the status and counter words of the call and fills the powers
+// rhop[n] = rho^n, n = 0..nmax, of the one radius ratio rho (1 + drho)
+// of the call (drho: its relative rounding error).  Latency-bound: chains
+// of some hundred dependent operations whatever the sizes (with the series
+// by nested double-double divisions the kernel took 13 us).
+// ---------------------------------------------------------------------------
+namespace
+{
+
+constexpr int POW_STRETCH = 8;
+
+// (mantissa, exponent) of a dd, the mantissa in [1, 2)
+struct ddx
+{
+    dd v;
+    int e;
+};
+
+__device__ __forceinline__ ddx ddx_norm(dd v, int e)
+{
+    const int h = ((__double2hiint(v.hi) >> 20) & 0x7ff) - 1023;
+    if (h == -1023)
+        return {dd{0.0, 0.0}, 0};
+    const double f = pow2i(-h);
+    return {dd{v.hi * f, v.lo * f}, e + h};
+}
+
+__device__ __forceinline__ ddx ddx_mul(ddx a, ddx b)
+{
+    return ddx_norm(dd_mul(a.v, b.v), a.e + b.e);
+}
+
+__device__ ddx ddx_pow(ddx b, long long k)
+{
+    ddx r{dd{1.0, 0.0}, 0};
+    while (k)
+    {
+        if (k & 1)
+            r = ddx_mul(r, b);
+        k >>= 1;
+        if (k)
+            b = ddx_mul(b, b);
+    }
+    return r;
+}
+
+} // namespace
+
+__global__ void k_geometry(GeometryArgs G)
+{
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (blockIdx.y == 0)
+    {
+        if (blockIdx.x == 0 && threadIdx.x < GEO_CLEAR_WORDS)
+            G.clear[threadIdx.x] = 0u;
+        if (G.rhop)
+            for (long long n = p; n <= G.nmax;
+                 n += (long long)gridDim.x * blockDim.x)
+            {
+                const ddx v = ddx_pow(
+                    ddx_norm(dd_fast(G.rho, G.rho * G.drho), 0), n);
+                G.rhop[n] = scalbn(v.v.hi, v.e);
+            }
+    }
+    if (p >= G.npairs)
+        return;
+    // sin h / h and cos h at h = lat / 8 (h^2 < 0.04): the terms from h^6 on
+    // in double (below 2^-26, so good to 2^-79), the first two in
+    // double-double; 1/6, 1/120, 1/2, 1/24 as sums of two doubles
+    const double h = 0.125 * G.lat[p];
+    const dd h2 = dd_mul(dd{h, 0.0}, dd{h, 0.0});
+    const double w = h2.hi;
+    const double ts =
+        fma(w, fma(w, fma(w, fma(w, fma(w, -1.0 / 1307674368000.0,
+                                        1.0 / 6227020800.0),
+                                 -1.0 / 39916800.0),
+                          1.0 / 362880.0),
+                   -1.0 / 5040.0),
+            0.0);
+    const double tc =
+        fma(w, fma(w, fma(w, fma(w, fma(w, -1.0 / 87178291200.0,
+                                        1.0 / 479001600.0),
+                                 -1.0 / 3628800.0),
+                          1.0 / 40320.0),
+                   -1.0 / 720.0),
+            0.0);
+    const dd one{1.0, 0.0};
+    dd s = dd_add(dd{1.0 / 120.0, 0x1.1111111111111p-63}, dd{ts, 0.0});
+    dd c = dd_add(dd{1.0 / 24.0, 0x1.5555555555555p-59}, dd{tc, 0.0});
+    s = dd_add(dd{-1.0 / 6.0, -0x1.5555555555555p-57}, dd_mul(h2, s));
+    c = dd_add(dd{-0.5, 0.0}, dd_mul(h2, c));
+    s = dd_add(one, dd_mul(h2, s));
+    c = dd_add(one, dd_mul(h2, c));
+    s = dd_mul(s, dd{h, 0.0});
+    for (int j = 0; j < 3; j++)
+    {
+        const dd s2 = dd_mul(s, s);
+        s = dd_mul(s, c);
+        s = dd{2.0 * s.hi, 2.0 * s.lo};
+        c = dd_add(one, dd{-2.0 * s2.hi, -2.0 * s2.lo});
+    }
+    if (blockIdx.y == 0)
+    {
+        G.t[p] = s.hi;
+        G.u[p] = c.hi;
+        G.z[p] = p < G.polar ? -dd_mul(c, c).hi : dd_mul(s, s).hi;
+        return;
+    }
+    const int e0 = (int)(blockIdx.y - 1) * POW_STRETCH;
+    const int e1 = min(e0 + POW_STRETCH, G.npow);
+    const ddx u = ddx_norm(c, 0);
+    // the first POW_LOW entries u^e, then u^(POW_LOW j)
+    ddx step = u, v;
+    if (e0 < POW_LOW)
+        v = ddx_pow(u, e0);
+    else
+    {
+        step = ddx_pow(u, POW_LOW);
+        v = ddx_pow(step, e0 - POW_LOW);
+    }
+    for (int e = e0; e < e1; e++)
+    {
+        G.pw[(size_t)e * G.npairs + p] = make_double2(v.v.hi, (double)v.e);
+        v = ddx_mul(v, step);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// Coefficients of one set in the recurrences' normalisations.  For every
+// (order, l) the two-degree pairs
+//     (k_l (eps C_m+2l + eps C_m+2l+2), the same of S),  (k_l C_m+2l+1, ..),
+// and, with cs not null, the one-degree (ct C, ct S) (leg.cuh).  Degrees
+// above nmax and S_n0 count as zero; rhop (or null) multiplies degree n
+// first, dr the factors of a radial derivative.
+// Layouts of the degree-ntab tables.  Memory-bound, one pass.
+// ---------------------------------------------------------------------------
+__global__ void k_two_scale(ScaleArgs A, long long m_lo)
+{
+    const long long m = m_lo + blockIdx.x;
+    const long long nmax = A.nmax;
+    if (m > nmax)
+        return;
+    const long long c0 = two_col0(A.ntab, m);
+    const long long t0 = tri_col0(A.ntab, m) - m;
+    const long long s0 = tri_col0(A.shc_nmax, m) - m;
+    const long long nl = two_len(nmax, m);
+    const long long TL = two_sum(A.ntab);
+    auto get = [&](long long n) {
+        if (n > nmax)
+            return make_double2(0.0, 0.0);
+        const double w = A.rhop ? A.rhop[n] : 1.0;
+        return make_double2(w * A.c[s0 + n], m == 0 ? 0.0 : w * A.s[s0 + n]);
+    };
+    auto amp = [&](long long n) {
+        double w = 1.0;
+        if (A.dr >= 1)
+            w *= (double)(n + 1);
+        if (A.dr >= 2)
+            w *= (double)(n + 2);
+        return w;
+    };
+    for (long long l = threadIdx.x; l < nl; l += blockDim.x)
+    {
+        const long long n = m + 2 * l;
+        const double2 e0 = get(n), o = get(n + 1), e1 = get(n + 2);
+        if (A.cs)
+        {
+            const double k0 = A.tc[t0 + n] * amp(n);
+            A.cs[t0 + n] = make_double2(k0 * e0.x, k0 * e0.y);
+            if (n < nmax)
+            {
+                const double k1 = A.tc[t0 + n + 1] * amp(n + 1);
+                A.cs[t0 + n + 1] = make_double2(k1 * o.x, k1 * o.y);
+            }
+        }
+        double a1 = A.kw[c0 + l], a2 = A.kw[TL + c0 + l],
+               a3 = A.kw[2 * TL + c0 + l];
+        if (A.dr > 0)
+        {
+            a1 *= amp(n);
+            a3 *= amp(n + 1);
+            a2 *= amp(n + 2);
+        }
+        A.cs2[2 * (c0 + l)] = make_double2(fma(a1, e0.x, a2 * e1.x),
+                                           fma(a1, e0.y, a2 * e1.y));
+        A.cs2[2 * (c0 + l) + 1] = make_double2(a3 * o.x, a3 * o.y);
+    }
+}
+
+cudaError_t launch_two_tables(long long nmax, const double *sg, double2 *ab,
+                              double2 *ag, double *kw, double *sm,
+                              cudaStream_t st)
+{
+    k_two_tables<<<(unsigned)(nmax + 1), TAB_THREADS, 0, st>>>(
+        nmax, sg, ab, ag, kw, sm, two_sum(nmax));
+    return cudaGetLastError();
+}
+
+cudaError_t launch_geometry(const GeometryArgs &G, cudaStream_t st)
+{
+    const int threads = 64;
+    const long long n = G.npairs > 0 ? G.npairs : 1;
+    const dim3 grid((unsigned)((n + threads - 1) / threads),
+                    1 + (unsigned)((G.npow + POW_STRETCH - 1) / POW_STRETCH));
+    k_geometry<<<grid, threads, 0, st>>>(G);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_two_scale(const ScaleArgs &A, long long m_lo,
+                             long long m_hi, cudaStream_t st)
+{
+    if (m_hi <= m_lo)
+        return cudaSuccess;
+    k_two_scale<<<(unsigned)(m_hi - m_lo), 128, 0, st>>>(A, m_lo);
+    return cudaGetLastError();
+}
+
+} // namespace cb

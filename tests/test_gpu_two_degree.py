@@ -1,0 +1,124 @@
+"""The two-degree recurrence (two.cuh) and the rules that choose it, against
+the CPU oracle: degrees around the rule's lower end, whole and partial
+32-pair groups, latitudes either side of its equatorial band, every radius
+rule and latitude orders it must leave to the one-degree kernels.
+
+Tolerance.  Either side's functions of degree n at a rounded latitude are off
+by about n 2^-53 / sin or cos(lat) relative to their size (the latitude's
+rounding acts as a phase n dlat); over a grid that averages to a small
+multiple of n 2^-53, and two independent sides with sums of random
+coefficients stay below 4 n 2^-53 in relative RMS.  The model has no degree-0
+term, so nothing hides in it."""
+import numpy as np
+import pytest
+
+from charm_b200.workloads import GM, R_EARTH, coef_rel_rms, kaula, rel_rms
+from oracle import orc
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def cb():
+    import charm_b200
+    return charm_b200
+
+
+def tol(n):
+    return 4.0 * n * 2.0 ** -53
+
+
+def model(n, seed):
+    c, s = kaula(n, seed)
+    c[0] = 0.0
+    return c, s
+
+
+def both(cb, p, g, n, kind=None, seed=7):
+    c, s = model(n, seed)
+    shc = cb.Shc(n, GM, R_EARTH, c, s)
+    f = cb.shs_point(p, shc, n) if kind is None else cb.shs_point_guru(
+        p, shc, n, *kind)
+    o = orc.Shc(n, GM, R_EARTH, c, s)
+    ref = orc.shs_point(g, o, n) if kind is None else orc.shs_point(g, o, n,
+                                                                    kind)
+    return np.asarray(f).ravel(), np.asarray(ref[0]).ravel()
+
+
+def grids(cb, name, n, r):
+    if name == "gl":
+        return cb.PointGridGL(n, r), orc.gl(n, r)
+    kind = orc.DH1 if name == "dh1" else orc.DH2
+    ctor = cb.PointGridDH1 if name == "dh1" else cb.PointGridDH2
+    return ctor(n, r), orc.dh(n, r, kind)
+
+
+@pytest.mark.parametrize("name", ["gl", "dh1", "dh2"])
+@pytest.mark.parametrize("nmax", [127, 128, 129, 191, 258])
+def test_synthesis(cb, name, nmax):
+    p, g = grids(cb, name, nmax, R_EARTH)
+    f, ref = both(cb, p, g, nmax)
+    assert rel_rms(f, ref) <= tol(nmax)
+
+
+# one radius above and below the sphere (folded into the coefficients), and
+# one so far that the powers would leave the range (general path)
+@pytest.mark.parametrize("ratio", [1.04, 0.98, 8.0])
+@pytest.mark.parametrize("kind", [None, (1, 0, 0), (2, 0, 0), (0, 0, 1),
+                                  (0, 0, 2), (1, 0, 1)])
+def test_radii_and_radial_derivatives(cb, ratio, kind):
+    n = 210
+    p, g = grids(cb, "gl", n, R_EARTH * ratio)
+    f, ref = both(cb, p, g, n, kind)
+    keep = np.repeat(np.abs(p.lat) < np.deg2rad(89.0), p.lon.size)
+    assert rel_rms(f[keep], ref[keep]) <= 4 * tol(n)
+
+
+@pytest.mark.parametrize("case", ["ascending", "regional", "shuffled",
+                                  "radii", "equator", "polar"])
+def test_custom_latitudes(cb, case):
+    """Orders and spans of latitudes: those that the two-degree kernel takes
+    (symmetric, towards the equator) and those that it must not."""
+    n = 160
+    rng = np.random.default_rng(3)
+    half = np.sort(rng.uniform(0.003, 1.56, 75))[::-1]
+    lat = np.concatenate([half, -half[::-1]])
+    r = np.full(lat.size, R_EARTH)
+    if case == "ascending":
+        lat = lat[::-1].copy()
+    elif case == "regional":
+        lat = np.linspace(1.1, -0.4, 71)
+        r = np.full(lat.size, R_EARTH)
+    elif case == "shuffled":
+        lat = rng.permutation(lat)
+    elif case == "radii":
+        r = R_EARTH + 1e4 * np.abs(lat)
+    elif case == "equator":
+        lat = np.linspace(0.04, -0.04, 9)
+        r = np.full(lat.size, R_EARTH)
+    elif case == "polar":
+        half = np.linspace(1.5706, 1.2, 70)
+        lat = np.concatenate([half, -half[::-1]])
+        r = np.full(lat.size, R_EARTH)
+    lon = np.arange(2 * n + 2) * (np.pi / (n + 1))
+    f, ref = both(cb, cb.PointGrid(lat, lon, r),
+                  orc.Point(orc.GRID, lat, lon, r), n)
+    assert rel_rms(f, ref) <= tol(n)
+
+
+def test_columns_that_start_below_the_double_range(cb):
+    """nmax 1500 at latitudes whose sectorial values underflow for most
+    orders (down to 1e-4800), against the oracle's X-numbers; every row."""
+    n = 1500
+    half = np.deg2rad(np.concatenate([np.linspace(89.9, 80.0, 40),
+                                      np.linspace(79.0, 5.0, 30)]))
+    lat = np.concatenate([half, -half[::-1]])
+    lon = np.arange(3) * 0.7
+    r = np.full(lat.size, R_EARTH)
+    f, ref = both(cb, cb.PointGrid(lat, lon, r),
+                  orc.Point(orc.GRID, lat, lon, r), n)
+    f, ref = f.reshape(lat.size, 3), ref.reshape(lat.size, 3)
+    rms = np.sqrt(np.mean(ref ** 2))
+    # next to the pole a rounding of the latitude is a phase n / cos(lat)
+    amp = 1.0 / np.cos(lat)
+    assert np.all(np.abs(f - ref).max(1) <= tol(n) * amp * rms)
