@@ -1239,19 +1239,38 @@ int choose_k_two(int n2)
     return best;
 }
 
-// Latitude pairs per lane of the analysis kernel.  Wider tiles amortise
-// the per-degree beta load and the transpose-reduce over more latitudes but
-// lower the resident warps (sha_grid.cu); CHARM_B200_SHA_K (1, 2, 4, 6 or
-// 8) overrides the choice for tuning.
-int choose_k_sha(long long npairs)
+// Latitude pairs per lane of the analysis kernels.  Wider tiles amortise
+// the per-degree table load and the transpose-reduce over more latitudes but
+// lower the resident warps (sha_grid.cu, sha_two.cu); CHARM_B200_SHA_K (1, 2,
+// 4, 6 or 8) overrides the choice for tuning.
+int choose_k_sha(long long npairs, bool two = false)
 {
     static const int forced = [] {
         const char *e = std::getenv("CHARM_B200_SHA_K");
         int k = e ? std::atoi(e) : 0;
-        return (k == 1 || k == 2 || k == 4 || k == 6 || k == 8) ? k : 0;
+        return (k >= 1 && k <= 8) ? k : 0;
     }();
-    if (forced)
+    if (forced && (two || forced <= 2 || forced % 2 == 0))
         return forced;
+    if (two)
+    {
+        // least padded work per step, 16 K issue cycles of the FP64 pipe and
+        // about 14 of the reduction; the widths above 5 (two or three warps
+        // per sub-partition) pay from the largest grids on only (nmax 2190:
+        // 0.92, 0.89, 0.91, 0.91 ms at K = 4..7, 5400: 11.7 .. 11.2 ms)
+        int best = 4, cost = 0;
+        for (int k = 4; k <= (npairs >= 2048 ? 7 : 5); k++)
+        {
+            const int t =
+                (int)((npairs + 32 * k - 1) / (32 * k)) * (16 * k + 14);
+            if (cost == 0 || t < cost)
+            {
+                cost = t;
+                best = k;
+            }
+        }
+        return best;
+    }
     if (npairs < 64)
         return 1;
     if (npairs < 1024)
@@ -1460,13 +1479,32 @@ struct GridGeo
     const int *row_n, *row_s;
     double *rhop = nullptr;
     unsigned *d_status = nullptr;
-    unsigned long long *counter = nullptr;   // counter[0], counter[8]
+    unsigned long long *counter = nullptr;
+    GeometryArgs args{};
+    bool pending = false;   // k_geometry not launched yet (geometry_launch)
 };
+
+Status geometry_launch(Context &c, GridGeo *G)
+{
+    Status st;
+    if (!G->pending)
+        return st;
+    G->pending = false;
+    Scope sc(c, TIMER_PREP);
+    CB_CUDA(launch_geometry(G->args, c.stream), st);
+    return st;
+}
 
 // Smallest degree of the two-degree recurrence: below it a call is bound by
 // launches and by the latency of one short column, not by the FP64 pipe
 // (nmax 95: 10.7 us with it, 10.9 us without, event timings).
 constexpr unsigned long TWO_MIN_NMAX = 128;
+// The same for the analysis, whose transpose-reduce weighs more the shorter
+// the columns are: degree and evaluated pairs (GL nmax 520, 700, 850: 53,
+// 72, 98 us against 44, 76, 119 with the one-degree kernel, and about 5 us
+// for the latitudes; DH1 520 58 against 68).
+constexpr unsigned long TWO_MIN_NMAX_SHA = 512;
+constexpr int TWO_MIN_PAIRS_SHA = 384;
 constexpr double TWO_NEAR = 0.05;      // |sin(lat)| (two.cuh)
 
 // Pairs that the two-degree recurrence may take: |lat| must not grow along
@@ -1512,7 +1550,7 @@ Status grid_geometry(Context &c, const charm_point *pnt, const Pairs &P,
     // host: lat, rho or weights (2), rows; device: the same, then t, u, z
     const size_t up = (size_t)np * (3 * 8 + 2 * 4);
     void *hp = nullptr;
-    CB_TRY(pinned(c, up, &hp));
+    CB_TRY(pinned(c, up + (size_t)np * 2 * 8, &hp));
     double *hlat = static_cast<double *>(hp);
     double *ha = hlat + np, *hb = ha + np;
     int *hrn = reinterpret_cast<int *>(hb + np);
@@ -1550,12 +1588,19 @@ Status grid_geometry(Context &c, const charm_point *pnt, const Pairs &P,
             G->r = r0;
         }
     }
-    if (allow_two && !G->rr && nmax >= TWO_MIN_NMAX)
+    if (allow_two && !G->rr &&
+        (weights ? nmax >= TWO_MIN_NMAX_SHA && np >= TWO_MIN_PAIRS_SHA
+                 : nmax >= TWO_MIN_NMAX))
         G->n2 = two_pairs(hlat, np, &G->polar);
+    // nothing for k_geometry to do but the sines: they come from the host
+    const bool plain = G->n2 == 0 && G->rho == 1.0;
+    if (plain)
+        for (int p = 0; p < np; p++)
+            sincos(hlat[p], &hlat[4 * np + p], &hlat[5 * np + p]);
     void *dgeo = nullptr;
     CB_TRY(buf(c, "geo", up + (size_t)np * 3 * 8, &dgeo));
-    CB_CUDA(cudaMemcpyAsync(dgeo, hp, up, cudaMemcpyHostToDevice, c.stream),
-            st);
+    CB_CUDA(cudaMemcpyAsync(dgeo, hp, up + (plain ? (size_t)np * 2 * 8 : 0),
+                            cudaMemcpyHostToDevice, c.stream), st);
     double *d = static_cast<double *>(dgeo);
     G->lat = d;
     G->rhos = G->w_n = d + np;
@@ -1571,6 +1616,11 @@ Status grid_geometry(Context &c, const charm_point *pnt, const Pairs &P,
     G->d_status = static_cast<unsigned *>(sp);
     G->counter = reinterpret_cast<unsigned long long *>(
         static_cast<char *>(sp) + 64);
+    if (plain)
+    {
+        CB_CUDA(cudaMemsetAsync(sp, 0, 256, c.stream), st);
+        return st;
+    }
     GeometryArgs A{};
     A.npairs = np;
     A.polar = G->polar;
@@ -1595,8 +1645,12 @@ Status grid_geometry(Context &c, const charm_point *pnt, const Pairs &P,
         A.rho = G->rho;
         A.drho = std::fma(-G->rho, r0, R) / r0 / G->rho;
     }
-    Scope sc(c, TIMER_PREP);
-    CB_CUDA(launch_geometry(A, c.stream), st);
+    G->args = A;
+    G->pending = true;
+    // the powers of the radius ratio enter the scaling of the coefficients,
+    // whose launch otherwise takes the geometry along; an analysis has none
+    if (G->rhop || weights)
+        CB_TRY(geometry_launch(c, G));
     return st;
 }
 
@@ -1642,11 +1696,12 @@ bool band_rows(const Pairs &P, int p0, int p1, int nlat, int r[4])
 
 // Bands of consecutive tiles (or tile groups) for the overlap of the grid's
 // host copies with the kernels: nb bands of units [u0, u1) of `units`, each
-// unit covering `per` latitude pairs; their row ranges in `rows`.  Returns
+// unit covering `per` latitude pairs; their row ranges in `rows`.  With
+// `tail`, pairs beyond the units' belong to the last band.  Returns
 // the number of bands, 1 when the rows do not split into contiguous
 // ranges.
 int grid_bands(const Pairs &P, int nlat, int units, int per, int nb,
-               std::vector<std::array<int, 6>> &bands)
+               std::vector<std::array<int, 6>> &bands, bool tail = false)
 {
     const int np = (int)P.row_n.size();
     bands.clear();
@@ -1657,7 +1712,8 @@ int grid_bands(const Pairs &P, int nlat, int units, int per, int nb,
     {
         const int u0 = (int)((long long)b * units / nb);
         const int u1 = (int)((long long)(b + 1) * units / nb);
-        const int p0 = std::min(np, u0 * per), p1 = std::min(np, u1 * per);
+        const int p0 = std::min(np, u0 * per);
+        const int p1 = tail && b == nb - 1 ? np : std::min(np, u1 * per);
         int r[4];
         if (p1 <= p0 || !band_rows(P, p0, p1, nlat, r))
         {
@@ -1774,7 +1830,11 @@ Status shs_grid(Context &c, const charm_point *pnt, const CoefIn &in,
         S.dr = dr;
         S.cs = dcs;
         S.cs2 = dcs2;
-        CB_CUDA(launch_scale_orders(S, m_lo, m_hi, c.stream), s2);
+        const bool with = G.pending && dcs2 && m_hi > m_lo;
+        CB_CUDA(launch_scale_orders(S, m_lo, m_hi, c.stream,
+                                    with ? &G.args : nullptr), s2);
+        if (with)
+            G.pending = false;
         return s2;
     };
     auto all_coefs = [&]() -> Status {
@@ -1814,6 +1874,8 @@ Status shs_grid(Context &c, const charm_point *pnt, const CoefIn &in,
         CB_TRY(row_fft_quarter(c, (long long)nlon, rf, &rfq));
     }
     unsigned *const d_status = G.d_status;
+    if (!coef_later)
+        CB_TRY(geometry_launch(c, &G));   // if the scaling did not take it
 
     ShsGridArgs A{};
     A.nmax = (long long)nmax;
@@ -1938,6 +2000,8 @@ Status shs_grid(Context &c, const charm_point *pnt, const CoefIn &in,
         CB_TRY(all_coefs());
         coef_later = false;
     }
+    if (!coef_later)
+        CB_TRY(geometry_launch(c, &G));
     if (nband > 1)
     {
         unsigned long long *bcnt = nullptr;
@@ -2288,9 +2352,14 @@ Status shs_batch(Context &c, const charm_point *pnt, size_t nsets,
         S.rhop = G.rhop;
         S.cs = cs_all ? cs_all + (size_t)j * T : nullptr;
         S.cs2 = cs2_all ? cs2_all + (size_t)j * T2 : nullptr;
+        const bool with = G.pending && S.cs2;
         Scope sc(c, TIMER_PREP);
-        CB_CUDA(launch_scale_orders(S, 0, S.nmax + 1, c.stream), st);
+        CB_CUDA(launch_scale_orders(S, 0, S.nmax + 1, c.stream,
+                                    with ? &G.args : nullptr), st);
+        if (with)
+            G.pending = false;
     }
+    CB_TRY(geometry_launch(c, &G));
     const RfftArgs *rf = nullptr, *rfq = nullptr;
     CB_TRY(row_fft(c, (long long)nlon, &rf));
     CB_TRY(row_fft_quarter(c, (long long)nlon, rf, &rfq));
@@ -3166,59 +3235,37 @@ Status sha_grid(Context &c, const charm_point *pnt, const double *f_host,
         }
     }
     const int np = (int)P.row_n.size();
-    size_t geo_bytes = (size_t)np * (4 * 8 + 2 * 4);
-    void *hp = nullptr;
-    CB_TRY(pinned(c, geo_bytes, &hp));
-    double *ht = static_cast<double *>(hp);
-    double *hu = ht + np;
-    double *hcn = hu + np;
-    double *hcs = hcn + np;
-    int *hrn = reinterpret_cast<int *>(hcs + np);
-    int *hrs = hrn + np;
-    for (int p = 0; p < np; p++)
-    {
-        double la = pnt->lat[P.row_n[p]];
-        sincos(la, &ht[p], &hu[p]);
-        hcn[p] = cq * pnt->w[P.row_n[p]];
-        hcs[p] = P.row_s[p] >= 0 ? cq * pnt->w[P.row_s[p]] : 0.0;
-        hrn[p] = P.row_n[p];
-        hrs[p] = P.row_s[p];
-    }
-    void *dgeo = nullptr;
-    CB_TRY(buf(c, "geo", geo_bytes, &dgeo));
-    CB_CUDA(cudaMemcpyAsync(dgeo, hp, geo_bytes, cudaMemcpyHostToDevice,
-                            c.stream), st);
-    const double *dt = static_cast<const double *>(dgeo);
-    const double *du = dt + np;
-    const double *dcn = du + np;
-    const double *dcsw = dcn + np;
-    const int *drn = reinterpret_cast<const int *>(dcsw + np);
-    const int *drs = drn + np;
+    GridGeo G;
+    CB_TRY(grid_geometry(c, pnt, P, nmax, R, true, true, cq, true, &G));
+    const int n2 = G.n2;
+    unsigned *const d_status = G.d_status;
 
     Tabs tab;
-    CB_TRY(tables(c, (long long)nmax, &tab));
+    CB_TRY(tables(c, (long long)nmax, &tab, n2 > 0));
 
     // work decomposition: K latitude pairs per lane, tiles of 32 K pairs,
-    // groups of tiles whose partial sums are added in fixed order
-    unsigned *d_status;
-    unsigned long long *d_counter;
-    CB_TRY(status_words(c, &d_status, &d_counter));
-    const int K = choose_k_sha(np);
-    const int ntiles = (np + 32 * K - 1) / (32 * K);
+    // groups of tiles whose partial sums are added in fixed order; with the
+    // two-degree kernel the pairs from n2 on are one more group
+    const int K = choose_k_sha(n2 > 0 ? n2 : np, n2 > 0);
+    const int ntiles = ((n2 > 0 ? n2 : np) + 32 * K - 1) / (32 * K);
     const long long T = (long long)(nmax + 1) * (nmax + 2) / 2;
     long long slots = (long long)c.num_sms * 8 * 4;
-    long long G = std::max<long long>(1, (2 * slots + nmax) / (nmax + 1));
-    G = std::min<long long>(G, ntiles);
+    long long Gn = std::max<long long>(1, (2 * slots + nmax) / (nmax + 1));
+    Gn = std::min<long long>(Gn, ntiles);
     // a host grid is analysed in bands of tiles, overlapped with its copy:
     // groups of single tiles (within 512 MB of partial sums) keep each
     // band's launch balanced (shorter work items)
     if (!d_fin)
-        G = std::max<long long>(
-            G, std::min<long long>(ntiles, (512LL << 20) / (16 * T)));
-    int tpg = (int)((ntiles + G - 1) / G);
-    G = (ntiles + tpg - 1) / tpg;
-    double2 *part = nullptr;
-    CB_TRY(dbuf(c, "sha_part", (size_t)G * T, &part));
+        Gn = std::max<long long>(
+            Gn, std::min<long long>(ntiles, (512LL << 20) / (16 * T)));
+    int tpg = (int)((ntiles + Gn - 1) / Gn);
+    Gn = (ntiles + tpg - 1) / tpg;
+    double2 *part = nullptr, *part1 = nullptr;
+    CB_TRY(dbuf(c, "sha_part",
+                (size_t)Gn * (n2 > 0 ? 2 * two_steps((long long)nmax) : T),
+                &part));
+    if (n2 > 0 && n2 < np)
+        CB_TRY(dbuf(c, "sha_part1", (size_t)T, &part1));
 
     // grid on the device and r2c along the parallels
     const double *fg = d_fin;
@@ -3267,25 +3314,79 @@ Status sha_grid(Context &c, const charm_point *pnt, const double *f_host,
     A.nmax = (long long)nmax;
     A.npairs = np;
     A.ntiles = ntiles;
-    A.ngroups = (int)G;
     A.tiles_per_group = tpg;
-    A.nitems = (long long)(nmax + 1) * G;
     A.tb = tab.tb;
     A.tmul = tab.tmul;
     A.ldmul = tab.ldmul;
     A.sg = tab.sg;
-    A.t = dt;
-    A.u = du;
-    A.row_n = drn;
-    A.row_s = drs;
-    A.cw_n = dcn;
-    A.cw_s = dcsw;
+    A.t = G.t;
+    A.u = G.u;
+    A.row_n = G.row_n;
+    A.row_s = G.row_s;
+    A.cw_n = G.w_n;
+    A.cw_s = G.w_s;
     A.F = F;
     A.ldF = ldF;
     A.part = part;
     A.polar_thr = polar_threshold(nmax);
-    A.counter = d_counter;
     A.status = d_status;
+    ShaTwoArgs B{};
+    B.nmax = (long long)nmax;
+    B.npairs = n2;
+    B.polar = G.polar;
+    B.ntiles = ntiles;
+    B.tiles_per_group = tpg;
+    B.ab = tab.ab;
+    B.ag = tab.ag;
+    B.sm = tab.sm;
+    B.tb = tab.tb;
+    B.tmul = tab.tmul;
+    B.ldmul = tab.ldmul;
+    B.sg = tab.sg;
+    B.t = G.t;
+    B.u = G.u;
+    B.z = G.z;
+    B.pw = G.pw;
+    B.pw_ld = np;
+    B.row_n = G.row_n;
+    B.row_s = G.row_s;
+    B.cw_n = G.w_n;
+    B.cw_s = G.w_s;
+    B.F = F;
+    B.ldF = ldF;
+    B.part = part;
+    B.part1 = part1;
+    B.polar_thr = A.polar_thr;
+    B.status = d_status;
+    // analysis of the orders [m_lo, m_hi) over the groups [g0, g1), with
+    // `last` also over the equatorial pairs; cnt: a cleared counter
+    auto analyse = [&](int g0, int g1, bool last, long long m_lo,
+                       long long m_hi, unsigned long long *cnt) {
+        long long items = (m_hi - m_lo) * (g1 - g0);
+        if (n2 > 0 && last && n2 < np)
+            items += m_hi - m_lo;
+        const int blocks = (int)std::max<long long>(
+            1, std::min<long long>((items + 3) / 4, (long long)c.num_sms * 8));
+        if (n2 > 0)
+        {
+            ShaTwoArgs b = B;
+            b.near0 = n2;
+            b.nnear = last ? np - n2 : 0;
+            b.group0 = g0;
+            b.ngroups = g1 - g0;
+            b.m0 = m_lo;
+            b.nitems = items;
+            b.counter = cnt;
+            return launch_sha_two(b, K, blocks, c.stream);
+        }
+        ShaGridArgs a = A;
+        a.group0 = g0;
+        a.ngroups = g1 - g0;
+        a.m0 = m_lo;
+        a.nitems = items;
+        a.counter = cnt;
+        return launch_sha_grid(a, K, blocks, c.stream);
+    };
 
     // rescaling from r0 to the coefficients' radius
     // (src/sha/sha_point.c:1088-1108 with src/shc/shc_rescale.c)
@@ -3317,6 +3418,27 @@ Status sha_grid(Context &c, const charm_point *pnt, const double *f_host,
         oc = dout;
         os = dout + Ts;
     }
+    // the caller's orders [m_lo, m_hi) from the partial sums
+    auto reduce = [&](long long m_lo, long long m_hi) {
+        if (n2 > 0)
+        {
+            TwoReduceArgs r{};
+            r.nmax = (long long)nmax;
+            r.shc_nmax = (long long)sn;
+            r.ngroups = (int)Gn;
+            r.part = part;
+            r.part1 = part1;
+            r.tc = tab.tc;
+            r.kw = tab.kw;
+            r.rescale = dres;
+            r.c = oc;
+            r.s = os;
+            return launch_two_reduce(r, m_lo, m_hi, c.stream);
+        }
+        return launch_sha_reduce_orders((long long)nmax, (long long)sn,
+                                        (int)Gn, T, part, tab.tc, dres, 1.0,
+                                        oc, os, m_lo, m_hi, c.stream);
+    };
 
     // Host input through the row transform: bands of tile groups; band b's
     // rows are copied (copy stream) while band b - 1 is transformed and
@@ -3325,10 +3447,10 @@ Status sha_grid(Context &c, const charm_point *pnt, const double *f_host,
     // each reduced and copied to the host (copy stream) while the next one
     // is analysed.
     std::vector<std::array<int, 6>> bands;
-    const int nband = (fdev && rf) ? grid_bands(P, (int)nlat, (int)G,
+    const int nband = (fdev && rf) ? grid_bands(P, (int)nlat, (int)Gn,
                                                 32 * K * tpg,
-                                                G >= 3 ? SHA_LAT_BANDS : 2,
-                                                bands)
+                                                Gn >= 3 ? SHA_LAT_BANDS : 2,
+                                                bands, n2 > 0)
                                    : 1;
     bool ordered = false;
     if (nband > 1)
@@ -3385,19 +3507,12 @@ Status sha_grid(Context &c, const charm_point *pnt, const double *f_host,
             const bool split = b == nband - 1 && nob > 1;
             for (int k = 0; k < (split ? nob : 1); k++)
             {
-                ShaGridArgs Ab = A;
-                Ab.group0 = bd[0];
-                Ab.ngroups = bd[1] - bd[0];
-                Ab.m0 = split ? mb[k] : 0;
-                Ab.nitems = (long long)(split ? mb[k + 1] - mb[k]
-                                              : (long long)nmax + 1) *
-                            Ab.ngroups;
-                Ab.counter = bcnt + (split ? nband + k : b);
-                const int gb = (int)std::min<long long>(
-                    (Ab.nitems + 3) / 4, (long long)c.num_sms * 8);
                 {
                     Scope sc(c, TIMER_SHA);
-                    CB_CUDA(launch_sha_grid(Ab, K, std::max(gb, 1), c.stream),
+                    CB_CUDA(analyse(bd[0], bd[1], b == nband - 1,
+                                    split ? mb[k] : 0,
+                                    split ? mb[k + 1] : (long long)nmax + 1,
+                                    bcnt + (split ? nband + k : b)),
                             st);
                 }
                 if (split)
@@ -3407,11 +3522,7 @@ Status sha_grid(Context &c, const charm_point *pnt, const double *f_host,
                     const long long m_hi =
                         k == nob - 1 ? (long long)sn + 1 : mb[k + 1];
                     Scope sc(c, TIMER_PREP);
-                    CB_CUDA(launch_sha_reduce_orders(
-                                (long long)nmax, (long long)sn, (int)G, T,
-                                part, tab.tc, dres, 1.0, oc, os, mb[k], m_hi,
-                                c.stream),
-                            st);
+                    CB_CUDA(reduce(mb[k], m_hi), st);
                     CB_CUDA(cudaEventRecord(c.band_ev[EV_ORD0 + k], c.stream), st);
                 }
             }
@@ -3449,10 +3560,9 @@ Status sha_grid(Context &c, const charm_point *pnt, const double *f_host,
         }
         else
             CB_TRY(rows_fft(0, (int)nlat));
-        int grid = (int)std::min<long long>((A.nitems + 3) / 4,
-                                            (long long)c.num_sms * 8);
         Scope sc(c, TIMER_SHA);
-        CB_CUDA(launch_sha_grid(A, K, std::max(grid, 1), c.stream), st);
+        CB_CUDA(analyse(0, (int)Gn, true, 0, (long long)nmax + 1, G.counter),
+                st);
     }
 
     if (ordered)
@@ -3462,9 +3572,7 @@ Status sha_grid(Context &c, const charm_point *pnt, const double *f_host,
     }
     {
         Scope sc(c, TIMER_PREP);
-        CB_CUDA(launch_sha_reduce((long long)nmax, (long long)sn, (int)G, T,
-                                  part, tab.tc, dres, 1.0, oc, os, c.stream),
-                st);
+        CB_CUDA(reduce(0, (long long)sn + 1), st);
     }
     if (!d_c)
     {

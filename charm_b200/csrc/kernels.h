@@ -178,6 +178,50 @@ struct ShaGridArgs
     double R;              // reference radius of the coefficients
 };
 
+// Grid analysis with the two-degree recurrence (sha_two.cu); fields as
+// ShaGridArgs and ShsTwoArgs.
+struct ShaTwoArgs
+{
+    long long nmax;
+    int npairs;            // pairs [0, npairs): two-degree recurrence
+    int polar;
+    int near0, nnear;      // pairs of the order's one-degree column
+    int ntiles;
+    int ngroups;           // tile groups of this launch
+    int group0;
+    long long m0;
+    int tiles_per_group;
+    long long nitems;      // orders x (ngroups + 1 if nnear > 0)
+    const double2 *ab, *ag;
+    const double *sm;
+    const double2 *tb;     // one-degree tables
+    const double *tmul;
+    int ldmul;
+    const double *sg;
+    const double *t, *u, *z;
+    const double2 *pw;
+    int pw_ld;
+    const int *row_n, *row_s;
+    const double *cw_n, *cw_s;
+    const double2 *F;
+    int ldF;
+    double2 *part;         // [groups][steps][even, odd] (C, S) sums
+    double2 *part1;        // [T] sums of the one-degree column
+    double polar_thr;
+    unsigned long long *counter;
+    unsigned *status;
+};
+
+struct TwoReduceArgs
+{
+    long long nmax, shc_nmax;
+    int ngroups;
+    const double2 *part, *part1;   // part1 null: no one-degree column
+    const double *tc, *kw;
+    const double *rescale;         // per degree, or null
+    double *c, *s;
+};
+
 // Block-mean values in cells (cell.cu).  Grid synthesis and analysis run
 // over pairs of cell rows (a northern row and its mirror [-latmax,
 // -latmin], or a row alone); scattered synthesis over single cells.
@@ -347,7 +391,8 @@ cudaError_t launch_tables(long long nmax, const double *r, const double *ri,
 // k_scale_cs for the orders [m_lo, m_hi) only
 // orders [m_lo, m_hi) in the forms A asks for
 cudaError_t launch_scale_orders(const ScaleArgs &A, long long m_lo,
-                                long long m_hi, cudaStream_t st);
+                                long long m_hi, cudaStream_t st,
+                                const GeometryArgs *G = nullptr);
 cudaError_t launch_scale_cs(long long nmax, long long shc_nmax,
                             const double *c, const double *s,
                             const double *tc, double2 *cs, cudaStream_t st);
@@ -382,12 +427,21 @@ cudaError_t launch_two_tables(long long nmax, const double *sg, double2 *ab,
                               cudaStream_t st);
 cudaError_t launch_geometry(const GeometryArgs &G, cudaStream_t st);
 // orders [m_lo, m_hi); A.cs2 must not be null
+// (G not null: the blocks of launch_geometry in the same launch; G->rhop
+// must be null)
 cudaError_t launch_two_scale(const ScaleArgs &A, long long m_lo,
-                             long long m_hi, cudaStream_t st);
+                             long long m_hi, const GeometryArgs *G,
+                             cudaStream_t st);
 // K latitude pairs per lane, 1..8; near tiles hold SHS_NEAR_PAIRS pairs
 constexpr int SHS_NEAR_PAIRS = 32;
 cudaError_t launch_shs_two(const ShsTwoArgs &A, int K, int grid,
                            cudaStream_t st);
+// K latitude pairs per lane, 1..8
+cudaError_t launch_sha_two(const ShaTwoArgs &A, int K, int grid,
+                           cudaStream_t st);
+// orders [m_lo, m_hi) of the caller's triangles
+cudaError_t launch_two_reduce(const TwoReduceArgs &A, long long m_lo,
+                              long long m_hi, cudaStream_t st);
 cudaError_t launch_gl_nodes(unsigned long nmax, double *lat, double *w,
                             unsigned *status, cudaStream_t st);
 cudaError_t launch_dh_nodes(unsigned long nmax, double *lat, double *w,

@@ -212,12 +212,13 @@ cudaError_t launch_scale_cs(long long nmax, long long shc_nmax,
 }
 
 cudaError_t launch_scale_orders(const ScaleArgs &A, long long m_lo,
-                                long long m_hi, cudaStream_t st)
+                                long long m_hi, cudaStream_t st,
+                                const GeometryArgs *G)
 {
     if (m_hi <= m_lo)
         return cudaSuccess;
     if (A.cs2)
-        return launch_two_scale(A, m_lo, m_hi, st);
+        return launch_two_scale(A, m_lo, m_hi, G, st);
     k_scale_cs<<<(int)(m_hi - m_lo), 128, 0, st>>>(
         A.ntab, A.nmax, A.shc_nmax, A.c, A.s, A.tc, A.rhop, A.cs, m_lo);
     return cudaGetLastError();

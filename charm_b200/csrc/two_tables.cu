@@ -133,7 +133,7 @@ __global__ void k_two_tables(long long nmax, const double *sg, double2 *ab,
 // ---------------------------------------------------------------------------
 // Latitudes.  Per pair, from the double-double sine and cosine of its
 // latitude (Taylor series of lat / 8, doubled three times): t, u rounded;
-// z = x2, or -u2 for the pairs below `polar`; and (blockIdx.y > 0) the power
+// z = x2, or -u2 for the pairs below `polar`; and (by > 0) the power
 // table of two_seed, POW_STRETCH entries per thread.  The first block also
 // clears the status and counter words of the call and fills the powers
 // rhop[n] = rho^n, n = 0..nmax, of the one radius ratio rho (1 + drho)
@@ -145,6 +145,17 @@ namespace
 {
 
 constexpr int POW_STRETCH = 8;
+constexpr int GEO_THREADS = 128;
+
+__host__ __device__ __forceinline__ int geo_blocks_x(const GeometryArgs &G)
+{
+    return G.npairs > 0 ? (G.npairs + GEO_THREADS - 1) / GEO_THREADS : 1;
+}
+
+__host__ __device__ __forceinline__ int geo_blocks_y(const GeometryArgs &G)
+{
+    return 1 + (G.npow + POW_STRETCH - 1) / POW_STRETCH;
+}
 
 // (mantissa, exponent) of a dd, the mantissa in [1, 2)
 struct ddx
@@ -183,16 +194,16 @@ __device__ ddx ddx_pow(ddx b, long long k)
 
 } // namespace
 
-__global__ void k_geometry(GeometryArgs G)
+__device__ void geometry_block(const GeometryArgs &G, int bx, int by)
 {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (blockIdx.y == 0)
+    const int p = bx * GEO_THREADS + (int)threadIdx.x;
+    if (by == 0)
     {
-        if (blockIdx.x == 0 && threadIdx.x < GEO_CLEAR_WORDS)
+        if (bx == 0 && threadIdx.x < GEO_CLEAR_WORDS)
             G.clear[threadIdx.x] = 0u;
         if (G.rhop)
             for (long long n = p; n <= G.nmax;
-                 n += (long long)gridDim.x * blockDim.x)
+                 n += (long long)geo_blocks_x(G) * GEO_THREADS)
             {
                 const ddx v = ddx_pow(
                     ddx_norm(dd_fast(G.rho, G.rho * G.drho), 0), n);
@@ -236,14 +247,14 @@ __global__ void k_geometry(GeometryArgs G)
         s = dd{2.0 * s.hi, 2.0 * s.lo};
         c = dd_add(one, dd{-2.0 * s2.hi, -2.0 * s2.lo});
     }
-    if (blockIdx.y == 0)
+    if (by == 0)
     {
         G.t[p] = s.hi;
         G.u[p] = c.hi;
         G.z[p] = p < G.polar ? -dd_mul(c, c).hi : dd_mul(s, s).hi;
         return;
     }
-    const int e0 = (int)(blockIdx.y - 1) * POW_STRETCH;
+    const int e0 = (by - 1) * POW_STRETCH;
     const int e1 = min(e0 + POW_STRETCH, G.npow);
     const ddx u = ddx_norm(c, 0);
     // the first POW_LOW entries u^e, then u^(POW_LOW j)
@@ -262,6 +273,11 @@ __global__ void k_geometry(GeometryArgs G)
     }
 }
 
+__global__ void k_geometry(GeometryArgs G)
+{
+    geometry_block(G, (int)blockIdx.x, (int)blockIdx.y);
+}
+
 // ---------------------------------------------------------------------------
 // Coefficients of one set in the recurrences' normalisations.  For every
 // (order, l) the two-degree pairs
@@ -269,11 +285,20 @@ __global__ void k_geometry(GeometryArgs G)
 // and, with cs not null, the one-degree (ct C, ct S) (leg.cuh).  Degrees
 // above nmax and S_n0 count as zero; rhop (or null) multiplies degree n
 // first, dr the factors of a radial derivative.
-// Layouts of the degree-ntab tables.  Memory-bound, one pass.
+// Layouts of the degree-ntab tables.  Memory-bound, one pass.  The first
+// `geo` blocks are k_geometry's (which a call without rhop does not have to
+// wait for): one launch and its latency less.
 // ---------------------------------------------------------------------------
-__global__ void k_two_scale(ScaleArgs A, long long m_lo)
+__global__ void k_two_scale(ScaleArgs A, long long m_lo, GeometryArgs G,
+                            int geo)
 {
-    const long long m = m_lo + blockIdx.x;
+    if ((int)blockIdx.x < geo)
+    {
+        const int nx = geo_blocks_x(G);
+        geometry_block(G, (int)blockIdx.x % nx, (int)blockIdx.x / nx);
+        return;
+    }
+    const long long m = m_lo + blockIdx.x - geo;
     const long long nmax = A.nmax;
     if (m > nmax)
         return;
@@ -335,20 +360,20 @@ cudaError_t launch_two_tables(long long nmax, const double *sg, double2 *ab,
 
 cudaError_t launch_geometry(const GeometryArgs &G, cudaStream_t st)
 {
-    const int threads = 64;
-    const long long n = G.npairs > 0 ? G.npairs : 1;
-    const dim3 grid((unsigned)((n + threads - 1) / threads),
-                    1 + (unsigned)((G.npow + POW_STRETCH - 1) / POW_STRETCH));
-    k_geometry<<<grid, threads, 0, st>>>(G);
+    const dim3 grid((unsigned)geo_blocks_x(G), (unsigned)geo_blocks_y(G));
+    k_geometry<<<grid, GEO_THREADS, 0, st>>>(G);
     return cudaGetLastError();
 }
 
 cudaError_t launch_two_scale(const ScaleArgs &A, long long m_lo,
-                             long long m_hi, cudaStream_t st)
+                             long long m_hi, const GeometryArgs *G,
+                             cudaStream_t st)
 {
     if (m_hi <= m_lo)
         return cudaSuccess;
-    k_two_scale<<<(unsigned)(m_hi - m_lo), 128, 0, st>>>(A, m_lo);
+    const int geo = G ? geo_blocks_x(*G) * geo_blocks_y(*G) : 0;
+    k_two_scale<<<(unsigned)(m_hi - m_lo + geo), GEO_THREADS, 0, st>>>(
+        A, m_lo, G ? *G : GeometryArgs{}, geo);
     return cudaGetLastError();
 }
 

@@ -122,3 +122,29 @@ def test_columns_that_start_below_the_double_range(cb):
     # next to the pole a rounding of the latitude is a phase n / cos(lat)
     amp = 1.0 / np.cos(lat)
     assert np.all(np.abs(f - ref).max(1) <= tol(n) * amp * rms)
+
+
+# either side of the rule's smallest grid (384 pairs, degree 512), whole and
+# partial tiles, degrees below the grid's, a triangle larger than the degree
+@pytest.mark.parametrize("name,grid_nmax,nmax", [
+    ("gl", 765, 765), ("gl", 766, 766), ("gl", 767, 511), ("gl", 800, 700),
+    ("dh1", 511, 511), ("dh1", 513, 513), ("dh2", 512, 512)])
+@pytest.mark.parametrize("height", [0.0, 5e3])
+def test_analysis(cb, name, grid_nmax, nmax, height):
+    r = R_EARTH + height
+    p, g = grids(cb, name, grid_nmax, r)
+    c, s = model(nmax, 11)
+    f = np.asarray(cb.shs_point(p, cb.Shc(nmax, GM, R_EARTH, c, s), nmax))
+    out = cb.sha_point(p, f, nmax, GM, r)
+    ref = orc.sha_point(g, f, nmax, GM, r)
+    assert coef_rel_rms(out.c, out.s, ref.c, ref.s) <= tol(nmax)
+    # every degree and order on its own scale: a wrong weight of one column
+    # or parity would hide in the whole
+    n = np.concatenate([np.arange(m, nmax + 1) for m in range(nmax + 1)])
+    size = np.sqrt(np.bincount(n, c ** 2 + s ** 2)) / np.sqrt(2.0 * np.arange(
+        nmax + 1) + 1.0)
+    size[:2] = size[2]
+    err = np.hypot(out.c - ref.c, out.s - ref.s)
+    assert np.all(err <= 200 * tol(nmax) * size[2])
+    high = (n > nmax // 2)
+    assert np.sqrt(np.mean(err[high] ** 2)) <= tol(nmax) * size[2]
