@@ -25,7 +25,8 @@ COMMON = ["-O3", "-std=c++17", "-lineinfo", "-ccbin", HOST_CXX,
           "-Xcompiler", "-fPIC,-fvisibility=hidden",
           "--expt-relaxed-constexpr"]
 
-SOURCES = ["tables.cu", "shs_grid.cu", "sha_grid.cu", "sctr.cu", "crd.cu", "probe.cu", "rfft.cu", "sha_static.cu", "f32.cu", "shs_tc.cu", "two_tables.cu", "shs_two.cu", "sha_two.cu", "cell.cu", "gfm.cu",
+SOURCES = ["tables.cu", "shs_grid.cu", "sha_grid.cu", "sctr.cu", "crd.cu", "probe.cu", "rfft.cu", "rfft_ct0.cu", "rfft_ct1.cu", "rfft_ct2.cu", "rfft_ct3.cu", "rfft_ct4.cu", "rfft_ct5.cu", "rfft_ct6.cu",
+           "sha_static.cu", "f32.cu", "shs_tc.cu", "two_tables.cu", "shs_two.cu", "sha_two.cu", "cell.cu", "gfm.cu",
            "engine.cpp", "capi.cpp"]
 
 

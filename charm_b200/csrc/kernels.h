@@ -342,6 +342,15 @@ struct ShaF32Args
 
 // Real <-> half-spectrum transforms of grid rows of even length L = 2H in
 // shared memory (rfft.cu).
+// One block of rows of a batched synthesis transform: output rows, spectra
+// and their last order.
+struct RfftRows
+{
+    double *x;
+    const double2 *X;
+    int kmax;
+};
+
 struct RfftArgs
 {
     long long nrows;
@@ -375,7 +384,20 @@ struct RfftArgs
     // the FFT_M value C l + q
     int C;
     const double2 *twM;
+    // synthesis of many row blocks in one launch (batch not null, on the
+    // device): entry b replaces x, X and kmax for the blocks blockIdx.y = b
+    const RfftRows *batch;
+    int nbatch;
 };
+
+// the plans of rfft_ct*.cu; cudaErrorInvalidConfiguration: not in the file
+cudaError_t launch_rfft_ct0(const RfftArgs &A, bool inverse, cudaStream_t st);
+cudaError_t launch_rfft_ct1(const RfftArgs &A, bool inverse, cudaStream_t st);
+cudaError_t launch_rfft_ct2(const RfftArgs &A, bool inverse, cudaStream_t st);
+cudaError_t launch_rfft_ct3(const RfftArgs &A, bool inverse, cudaStream_t st);
+cudaError_t launch_rfft_ct4(const RfftArgs &A, bool inverse, cudaStream_t st);
+cudaError_t launch_rfft_ct5(const RfftArgs &A, bool inverse, cudaStream_t st);
+cudaError_t launch_rfft_ct6(const RfftArgs &A, bool inverse, cudaStream_t st);
 
 // Size of the fixed device scratch of the allocation-free analysis
 // (sha_static.cu) and the largest degree it serves.
