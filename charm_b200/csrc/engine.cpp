@@ -1222,8 +1222,10 @@ int choose_k(int kgrad, int dlat, long long nunits)
 // another), 15 K + 6 issue cycles per step; narrow tiles for few latitudes,
 // where the items of wide ones would not fill the GPU (K = 1 fastest at 181
 // and 251 pairs, 2 at 501 and 721).
-int choose_k_two(int n2)
+int choose_k_two(int n2, int mode)
 {
+    if (mode > 0)
+        return n2 >= 320 ? 2 : 1;
     if (n2 <= 896)
         return n2 >= 320 ? 2 : 1;
     int best = 4, cost = 0;
@@ -1468,6 +1470,10 @@ Status coef_to_device(Context &c, const CoefIn &in, unsigned long nmax,
 struct GridGeo
 {
     int np = 0, n2 = 0, polar = 0;
+    // leading pairs at a pole (POLE_COS): the quantities with 1 / cos(lat)
+    // are rounding noise there, the same noise from every call only if one
+    // kernel forms it, the one-degree one
+    int npole = 0;
     // one radius r for all rows, other than R: (R / r)^n is folded into the
     // coefficients (rhop), the call's factor is GM / r^(dorder + 1), and rr
     // is false
@@ -1496,9 +1502,13 @@ Status geometry_launch(Context &c, GridGeo *G)
 }
 
 // Smallest degree of the two-degree recurrence: below it a call is bound by
-// launches and by the latency of one short column, not by the FP64 pipe
-// (nmax 95: 10.7 us with it, 10.9 us without, event timings).
+// launches and by the latency of one short column, not by the FP64 pipe.
+// With derivatives or several sets there is more work per column; the
+// potential of one set gains from about 400 on (kernel at GL nmax 360, 420,
+// 500: 20.8, 22.8, 26.9 us against 21.0, 25.7, 36.2, and 3 us for the second
+// form of the coefficients).
 constexpr unsigned long TWO_MIN_NMAX = 128;
+constexpr unsigned long TWO_MIN_NMAX_ONE = 400;
 // The same for the analysis, whose transpose-reduce weighs more the shorter
 // the columns are: degree and evaluated pairs (GL nmax 520, 700, 850: 53,
 // 72, 98 us against 44, 76, 119 with the one-degree kernel, and about 5 us
@@ -1506,6 +1516,7 @@ constexpr unsigned long TWO_MIN_NMAX = 128;
 constexpr unsigned long TWO_MIN_NMAX_SHA = 512;
 constexpr int TWO_MIN_PAIRS_SHA = 384;
 constexpr double TWO_NEAR = 0.05;      // |sin(lat)| (two.cuh)
+constexpr double POLE_COS = 1e-6;
 
 // Pairs that the two-degree recurrence may take: |lat| must not grow along
 // the pairs (so that neighbouring lanes are neighbouring latitudes and the
@@ -1537,12 +1548,13 @@ int two_pairs(const double *lat, int np, int *polar)
     return n2;
 }
 
-// wn, ws (analysis): the weights of the pairs' rows, or null.  r_eq: every
-// row at the coefficients' radius R (nothing to fold); allow_two: the call's
-// kernels exist in the two-degree form.
+// weights (analysis): the rows' quadrature weights times cw are uploaded too.
+// r_eq: every row at the coefficients' radius R (nothing to fold); two_min:
+// the least degree for the two-degree recurrence.
 Status grid_geometry(Context &c, const charm_point *pnt, const Pairs &P,
-                     unsigned long nmax, double R, bool r_eq, bool allow_two,
-                     double cw, bool weights, GridGeo *G)
+                     unsigned long nmax, double R, bool r_eq,
+                     unsigned long two_min, double cw, bool weights,
+                     GridGeo *G)
 {
     Status st;
     const int np = (int)P.row_n.size();
@@ -1588,18 +1600,22 @@ Status grid_geometry(Context &c, const charm_point *pnt, const Pairs &P,
             G->r = r0;
         }
     }
-    if (allow_two && !G->rr &&
-        (weights ? nmax >= TWO_MIN_NMAX_SHA && np >= TWO_MIN_PAIRS_SHA
-                 : nmax >= TWO_MIN_NMAX))
+    if (!G->rr && nmax >= two_min && (!weights || np >= TWO_MIN_PAIRS_SHA))
         G->n2 = two_pairs(hlat, np, &G->polar);
     // nothing for k_geometry to do but the sines: they come from the host
+    // (and for the pairs at a pole in any case, so that their noise is the
+    // same with and without it)
     const bool plain = G->n2 == 0 && G->rho == 1.0;
-    if (plain)
-        for (int p = 0; p < np; p++)
-            sincos(hlat[p], &hlat[4 * np + p], &hlat[5 * np + p]);
+    double *const ht = hlat + 4 * np, *const hu = hlat + 5 * np;
+    while (G->npole < np && std::fabs(hlat[G->npole]) >= PI / 2 - POLE_COS)
+        G->npole++;
+    for (int p = 0; p < (plain ? np : G->npole); p++)
+        sincos(hlat[p], &ht[p], &hu[p]);
     void *dgeo = nullptr;
     CB_TRY(buf(c, "geo", up + (size_t)np * 3 * 8, &dgeo));
-    CB_CUDA(cudaMemcpyAsync(dgeo, hp, up + (plain ? (size_t)np * 2 * 8 : 0),
+    CB_CUDA(cudaMemcpyAsync(dgeo, hp,
+                            up + (plain || G->npole > 0 ? (size_t)np * 2 * 8
+                                                        : 0),
                             cudaMemcpyHostToDevice, c.stream), st);
     double *d = static_cast<double *>(dgeo);
     G->lat = d;
@@ -1624,6 +1640,7 @@ Status grid_geometry(Context &c, const charm_point *pnt, const Pairs &P,
     GeometryArgs A{};
     A.npairs = np;
     A.polar = G->polar;
+    A.given = G->npole;
     A.lat = d;
     A.t = dt;
     A.u = dt + np;
@@ -1782,17 +1799,24 @@ Status shs_grid(Context &c, const charm_point *pnt, const CoefIn &in,
     int dorder, npar;
     mur_dorder(in.mu, in.r, kgrad, dr, dlat, dlon, &mur, &dorder, &npar);
 
-    // the two-degree recurrence serves the quantities without a latitudinal
-    // derivative
     GridGeo G;
     CB_TRY(grid_geometry(c, pnt, P, nmax, in.r, r_eq,
-                         kgrad == 0 && dlat == 0, 0.0, false, &G));
+                         kgrad > 0 || dlat > 0 ? TWO_MIN_NMAX
+                                               : TWO_MIN_NMAX_ONE,
+                         0.0, false, &G));
+    // ShsTwoArgs::mode and its coefficient families
+    const int mode = kgrad == 0 ? dlat : 2 + kgrad;
+    ScaleArgs fam{};
+    scale_families(&fam, mode);
     mur_dorder(in.mu, G.r, kgrad, dr, dlat, dlon, &mur, &dorder, &npar);
     const int n2 = G.n2;
 
     Tabs tab;
     CB_TRY(tables(c, (long long)nmax, &tab, n2 > 0));
-    const bool old_too = n2 < np;   // some latitudes on the one-degree path
+    // pairs whose rows the one-degree kernel forms again (GridGeo::npole)
+    const int npole = n2 > 0 && kgrad > 0 ? G.npole : 0;
+    // some latitudes on the one-degree path
+    const bool old_too = n2 < np || npole > 0;
     // Host coefficients of a call whose grid goes to the host are uploaded
     // later, in bands of orders overlapped with the synthesis of the first
     // band of latitudes (when the call runs in bands), else all now.
@@ -1805,10 +1829,11 @@ Status shs_grid(Context &c, const charm_point *pnt, const CoefIn &in,
         !in.dc && !d_f &&
         shs_k_settled(c, kgrad, dr, dlat, variant, (long long)nmax, np);
     if (old_too)
-        CB_TRY(dbuf(c, "cs", (size_t)((nmax + 1) * (nmax + 2) / 2), &dcs));
+        CB_TRY(dbuf(c, "cs", (size_t)((nmax + 1) * (nmax + 2) / 2) *
+                                 (n2 > 0 ? fam.nfam : 1), &dcs));
     if (n2 > 0)
-        CB_TRY(dbuf(c, "cs2", (size_t)(2 * two_steps((long long)nmax)),
-                    &dcs2));
+        CB_TRY(dbuf(c, "cs2", (size_t)(2 * two_steps((long long)nmax)) *
+                                  fam.nfam, &dcs2));
     if (!in.dc)
     {
         CB_TRY(dbuf(c, "shc_in", (size_t)(2 * Ts), &raw));
@@ -1819,7 +1844,7 @@ Status shs_grid(Context &c, const charm_point *pnt, const CoefIn &in,
     auto scale = [&](long long m_lo, long long m_hi) -> Status {
         Status s2;
         Scope sc(c, TIMER_PREP);
-        ScaleArgs S{};
+        ScaleArgs S = fam;
         S.ntab = S.nmax = (long long)nmax;
         S.shc_nmax = (long long)in.nmax;
         S.c = src_c;
@@ -1827,7 +1852,7 @@ Status shs_grid(Context &c, const charm_point *pnt, const CoefIn &in,
         S.tc = tab.tc;
         S.kw = tab.kw;
         S.rhop = G.rhop;
-        S.dr = dr;
+        S.dr = kgrad == 0 ? dr : 0;
         S.cs = dcs;
         S.cs2 = dcs2;
         const bool with = G.pending && dcs2 && m_hi > m_lo;
@@ -1899,6 +1924,7 @@ Status shs_grid(Context &c, const charm_point *pnt, const CoefIn &in,
     A.polar_thr = polar_threshold(nmax);
     A.status = d_status;
     ShsTwoArgs B{};
+    B.mode = mode;
     B.nmax = (long long)nmax;
     B.npairs = n2;
     B.polar = G.polar;
@@ -1949,7 +1975,19 @@ Status shs_grid(Context &c, const charm_point *pnt, const CoefIn &in,
             b.m0 = m_lo;
             b.nitems = (m_hi - m_lo) * (b.ntiles + b.near_tiles);
             b.counter = cnt;
-            return launch_shs_two(b, K, blocks(b.nitems), c.stream);
+            const cudaError_t e =
+                launch_shs_two(b, K, blocks(b.nitems), c.stream);
+            if (e != cudaSuccess || p0 > 0 || npole == 0)
+                return e;
+            // (the families' first one-degree form is C, S themselves)
+            ShsGridArgs a = A;
+            a.npairs = npole;
+            a.ntiles = (npole + 31) / 32;
+            a.m0 = m_lo;
+            a.nitems = (m_hi - m_lo) * a.ntiles;
+            a.counter = cnt + 16;
+            return launch_shs_grid(a, kgrad, dr, dlat, false, 1,
+                                   blocks(a.nitems), c.stream);
         }
         ShsGridArgs a = A;
         a.tile0 = p0 / (32 * K);
@@ -1960,12 +1998,12 @@ Status shs_grid(Context &c, const charm_point *pnt, const CoefIn &in,
         return launch_shs_grid(a, kgrad, dr, dlat, G.rr, K, blocks(a.nitems),
                                c.stream);
     };
-    int K = n2 > 0 ? choose_k_two(n2) : choose_k(kgrad, dlat, np);
+    int K = n2 > 0 ? choose_k_two(n2, mode) : choose_k(kgrad, dlat, np);
     // autotuned tile (first call of this shape)
     {
         auto trial = [&](int k) {
             const cudaError_t e = cudaMemsetAsync(
-                G.counter, 0, sizeof(unsigned long long), c.stream);
+                G.counter, 0, 17 * sizeof(unsigned long long), c.stream);
             return e != cudaSuccess ? e
                                     : synth(k, 0, np, 0, (long long)nmax + 1,
                                             G.counter);
@@ -1975,13 +2013,14 @@ Status shs_grid(Context &c, const charm_point *pnt, const CoefIn &in,
         std::vector<int> cands =
             kgrad >= 1 || dlat > 0 ? std::vector<int>{1, 2}
                                    : std::vector<int>{1, 2, 4};
-        if (n2 > 0)
+        if (n2 > 0 && mode == 0)
             cands = n2 <= 1024 ? std::vector<int>{1, 2, 3, 4, 5, 6}
                                : std::vector<int>{3, 4, 5, 6, 7, 8};
         CB_TRY(tune_shs_k(c, trial, cands, kgrad, dr, dlat, variant,
                           (long long)nmax, np, &K));
         if (timed)
-            CB_CUDA(cudaMemsetAsync(G.counter, 0, sizeof(unsigned long long),
+            CB_CUDA(cudaMemsetAsync(G.counter, 0,
+                                    17 * sizeof(unsigned long long),
                                     c.stream), st);
     }
 
@@ -2005,8 +2044,8 @@ Status shs_grid(Context &c, const charm_point *pnt, const CoefIn &in,
     if (nband > 1)
     {
         unsigned long long *bcnt = nullptr;
-        CB_TRY(dbuf(c, "band_counters", 16, &bcnt));
-        CB_CUDA(cudaMemsetAsync(bcnt, 0, 16 * sizeof(unsigned long long),
+        CB_TRY(dbuf(c, "band_counters", 32, &bcnt));
+        CB_CUDA(cudaMemsetAsync(bcnt, 0, 32 * sizeof(unsigned long long),
                                 c.stream), st);
         // orders in up to SHS_ORD_BANDS bands of about equal numbers of
         // coefficients
@@ -2375,16 +2414,22 @@ Status shs_batch(Context &c, const charm_point *pnt, size_t nsets,
     CB_TRY(batch_pairs(c, pnt, N, R, &BG));
     const int np = BG.np;
     GridGeo G;
-    CB_TRY(grid_geometry(c, pnt, BG.P, N, R, BG.r_eq,
-                         kgrad == 0 || kgrad == 3, 0.0, false, &G));
+    CB_TRY(grid_geometry(c, pnt, BG.P, N, R, BG.r_eq, TWO_MIN_NMAX, 0.0, false,
+                         &G));
     const int n2 = G.n2;
-    // the gradient kinds stay with the one-degree recurrence
-    const bool old_too = n2 < np || kgrad != 0;
+    const bool two = n2 > 0;
+    const int npole = two && kgrad > 0 ? G.npole : 0;
+    const bool old_too = n2 < np || npole > 0;
+    // ShsTwoArgs::mode (kgrad 3 forms all ten quantities in one pass)
+    ScaleArgs fam{};
+    const int mode = kgrad == 0 ? 0 : 2 + kgrad;
+    scale_families(&fam, mode);
 
     Tabs tab;
     CB_TRY(tables(c, (long long)N, &tab, n2 > 0));
-    const long long T = (long long)(N + 1) * (N + 2) / 2;
-    const long long T2 = 2 * two_steps((long long)N);
+    const long long T = (long long)(N + 1) * (N + 2) / 2 *
+                        (two ? fam.nfam : 1);
+    const long long T2 = 2 * two_steps((long long)N) * fam.nfam;
     double2 *cs_all = nullptr, *cs2_all = nullptr;
     if (old_too)
         CB_TRY(dbuf(c, "batch_cs", (size_t)nsets * T, &cs_all));
@@ -2392,7 +2437,7 @@ Status shs_batch(Context &c, const charm_point *pnt, size_t nsets,
         CB_TRY(dbuf(c, "batch_cs2", (size_t)nsets * T2, &cs2_all));
     for (size_t j = 0; j < nsets; j++)
     {
-        ScaleArgs S{};
+        ScaleArgs S = fam;
         S.ntab = (long long)N;
         S.nmax = (long long)nmax_v[j];
         S.shc_nmax = (long long)shc_nmax_v[j];
@@ -2424,20 +2469,24 @@ Status shs_batch(Context &c, const charm_point *pnt, size_t nsets,
     struct Kind
     {
         int kgrad, npar, base;
-        int slot[6];
+        int slot[10];
     };
     std::vector<Kind> kinds;
     const Kind K0{0, 1, 0, {0}};
     const Kind K1{1, 3, 0, {1, 2, 0}};
     const Kind K2{2, 6, 0, {3, 4, 1, 5, 2, 0}};
-    if (kgrad == 0 || kgrad == 3)
+    const Kind KT{3, 10, 0, {0, 2, 3, 1, 7, 8, 5, 9, 6, 4}};
+    const bool ten = two && kgrad == 3;
+    if (ten)
+        kinds.push_back(KT);
+    else if (kgrad == 0 || kgrad == 3)
         kinds.push_back(K0);
-    if (kgrad == 1 || kgrad == 3)
+    if (kgrad == 1 || (kgrad == 3 && !ten))
     {
         kinds.push_back(K1);
         kinds.back().base = kgrad == 3 ? 1 : 0;
     }
-    if (kgrad == 2 || kgrad == 3)
+    if (kgrad == 2 || (kgrad == 3 && !ten))
     {
         kinds.push_back(K2);
         kinds.back().base = kgrad == 3 ? 4 : 0;
@@ -2456,8 +2505,7 @@ Status shs_batch(Context &c, const charm_point *pnt, size_t nsets,
         BatchSet *dsets = nullptr;
         CB_TRY(dbuf(c, "batch_sets", bsz, &dsets));
         std::vector<BatchSet> hsets(bsz);
-        const bool two = kg == 0 && n2 > 0;
-        const int K = two ? choose_k_two(n2) : choose_k(kg, dd, np);
+        const int K = two ? choose_k_two(n2, mode) : choose_k(kg, dd, np);
         const int near = two ? (np - n2 + SHS_NEAR_PAIRS - 1) / SHS_NEAR_PAIRS
                              : 0;
         const int ntiles = ((two ? n2 : np) + 32 * K - 1) / (32 * K);
@@ -2470,8 +2518,16 @@ Status shs_batch(Context &c, const charm_point *pnt, size_t nsets,
                 const size_t j = j0 + b;
                 double mur;
                 int dorder, npar_j;
-                mur_dorder(mu_v[j], G.r, kg, dd, dd, dd, &mur, &dorder,
-                           &npar_j);
+                mur_dorder(mu_v[j], G.r, ten ? 0 : kg, ten ? 0 : dd,
+                           ten ? 0 : dd, ten ? 0 : dd, &mur, &dorder, &npar_j);
+                if (ten)
+                {
+                    int dk, nk;
+                    mur_dorder(mu_v[j], G.r, 1, 1, 1, 1, &hsets[b].mur1, &dk,
+                               &nk);
+                    mur_dorder(mu_v[j], G.r, 2, 2, 2, 2, &hsets[b].mur2, &dk,
+                               &nk);
+                }
                 hsets[b].nmax = (long long)nmax_v[j];
                 hsets[b].item0 = items;
                 hsets[b].cs1 = cs_all ? cs_all + j * T : nullptr;
@@ -2482,14 +2538,16 @@ Status shs_batch(Context &c, const charm_point *pnt, size_t nsets,
                 items += (long long)(nmax_v[j] + 1) * (ntiles + near);
             }
             CB_TRY(h2d_small(c, dsets, hsets.data(), nb * sizeof(BatchSet)));
-            CB_CUDA(cudaMemsetAsync(G.counter, 0, sizeof(unsigned long long),
-                                    c.stream), st);
+            CB_CUDA(cudaMemsetAsync(G.counter, 0,
+                                    20 * sizeof(unsigned long long), c.stream),
+                    st);
             const int grid = (int)std::max<long long>(
                 1, std::min<long long>((items + 3) / 4,
                                        (long long)c.num_sms * 8));
             if (two)
             {
                 ShsTwoArgs B{};
+                B.mode = mode;
                 B.nmax = (long long)N;
                 B.npairs = n2;
                 B.polar = G.polar;
@@ -2519,8 +2577,64 @@ Status shs_batch(Context &c, const charm_point *pnt, size_t nsets,
                 B.status = d_status;
                 B.sets = dsets;
                 B.nsets = (int)nb;
-                Scope sc(c, TIMER_SHS);
-                CB_CUDA(launch_shs_two(B, K, grid, c.stream), st);
+                {
+                    Scope sc(c, TIMER_SHS);
+                    CB_CUDA(launch_shs_two(B, K, grid, c.stream), st);
+                }
+                // the rows at a pole again (GridGeo::npole): grad1, grad2
+                for (int k = 1; k <= 2 && npole > 0; k++)
+                {
+                    if (kg != k && kg != 3)
+                        continue;
+                    const int tiles = (npole + 31) / 32;
+                    std::vector<BatchSet> pol(hsets.begin(),
+                                              hsets.begin() + nb);
+                    long long n = 0;
+                    for (BatchSet &h : pol)
+                    {
+                        h.item0 = n;
+                        h.cs = h.cs1;
+                        if (ten)
+                        {
+                            h.out += (size_t)(k == 1 ? 1 : 4) * nlat * ldf;
+                            h.mur = k == 1 ? h.mur1 : h.mur2;
+                        }
+                        n += (h.nmax + 1) * tiles;
+                    }
+                    BatchSet *dpol = nullptr;
+                    CB_TRY(dbuf(c, "batch_sets_pole" + std::to_string(k),
+                                bsz, &dpol));
+                    CB_TRY(h2d_small(c, dpol, pol.data(),
+                                     nb * sizeof(BatchSet)));
+                    ShsGridArgs A{};
+                    A.nmax = (long long)N;
+                    A.npairs = npole;
+                    A.ntiles = tiles;
+                    A.nitems = n;
+                    A.tb = tab.tb;
+                    A.tmul = tab.tmul;
+                    A.ldmul = tab.ldmul;
+                    A.sg = tab.sg;
+                    A.t = G.t;
+                    A.u = G.u;
+                    A.rho = G.rhos;
+                    A.row_n = G.row_n;
+                    A.row_s = G.row_s;
+                    A.nlat = (int)nlat;
+                    A.ldf = ldf;
+                    A.fft_pack = 1;
+                    A.dlon = k;
+                    A.counter = G.counter + 16 + k;
+                    A.status = d_status;
+                    A.sets = dpol;
+                    A.nsets = (int)nb;
+                    const int gp = (int)std::max<long long>(
+                        1, std::min<long long>((n + 3) / 4,
+                                               (long long)c.num_sms * 8));
+                    Scope sc(c, TIMER_SHS);
+                    CB_CUDA(launch_shs_grid(A, k, k, k, false, 1, gp,
+                                            c.stream), st);
+                }
             }
             else
             {
@@ -3254,7 +3368,8 @@ Status sha_grid(Context &c, const charm_point *pnt, const double *f_host,
     }
     const int np = (int)P.row_n.size();
     GridGeo G;
-    CB_TRY(grid_geometry(c, pnt, P, nmax, R, true, true, cq, true, &G));
+    CB_TRY(grid_geometry(c, pnt, P, nmax, R, true, TWO_MIN_NMAX_SHA, cq, true,
+                         &G));
     const int n2 = G.n2;
     unsigned *const d_status = G.d_status;
 

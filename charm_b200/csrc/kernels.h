@@ -28,6 +28,7 @@ struct BatchSet
     const double2 *cs1;   // one-degree form beside a two-degree cs
     double2 *out;
     double mur;
+    double mur1, mur2;    // of grad1 and grad2 beside the potential's mur
     double polar_thr;
 };
 
@@ -68,10 +69,13 @@ struct ShsGridArgs
     int nsets;
 };
 
-// Grid synthesis of the potential and its radial derivatives with the
-// two-degree recurrence (shs_two.cu, two.cuh); fields as ShsGridArgs.
+// Grid synthesis with the two-degree recurrence (shs_two.cu, two.cuh); fields
+// as ShsGridArgs.
 struct ShsTwoArgs
 {
+    // 0 potential and radial derivatives, 1 and 2 latitudinal derivatives,
+    // 3 grad1, 4 grad2, 5 all ten quantities (batched sets only)
+    int mode;
     long long nmax;
     int npairs;            // pairs [0, npairs) of the geometry arrays
     int polar;             // pairs below this take z = -cos^2 (multiple of 32)
@@ -113,6 +117,7 @@ struct GeometryArgs
 {
     int npairs;
     int polar;             // pairs below this store z = -cos^2, else sin^2
+    int given;             // pairs below this have t and u already
     const double *lat;
     double *t, *u, *z;
     double2 *pw;           // power table of two_seed, npow entries (or 0)
@@ -137,9 +142,13 @@ struct ScaleArgs
     const double *rhop;      // factor of degree n, or null
     int dr;                  // radial derivative order folded into cs2 (and
                              // into cs beside it)
-    double2 *cs;             // one-degree form, or null
-    double2 *cs2;            // two-degree form, or null
+    int nfam;                // families of the mode (shs_two.cu), X alone 1:
+    int fam[5];              // 0 X, 1 H, 2 N, 3 G, 4 J
+    double2 *cs;             // one-degree form [family][T], or null
+    double2 *cs2;            // two-degree form [family][2 steps], or null
 };
+// fills nfam, fam for a mode of ShsTwoArgs
+void scale_families(ScaleArgs *A, int mode);
 
 // Grid analysis: C_nm, S_nm partial sums per latitude group (sha_grid.cu).
 struct ShaGridArgs

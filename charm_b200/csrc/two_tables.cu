@@ -249,8 +249,11 @@ __device__ void geometry_block(const GeometryArgs &G, int bx, int by)
     }
     if (by == 0)
     {
-        G.t[p] = s.hi;
-        G.u[p] = c.hi;
+        if (p >= G.given)
+        {
+            G.t[p] = s.hi;
+            G.u[p] = c.hi;
+        }
         G.z[p] = p < G.polar ? -dd_mul(c, c).hi : dd_mul(s, s).hi;
         return;
     }
@@ -282,9 +285,11 @@ __global__ void k_geometry(GeometryArgs G)
 // Coefficients of one set in the recurrences' normalisations.  For every
 // (order, l) the two-degree pairs
 //     (k_l (eps C_m+2l + eps C_m+2l+2), the same of S),  (k_l C_m+2l+1, ..),
-// and, with cs not null, the one-degree (ct C, ct S) (leg.cuh).  Degrees
-// above nmax and S_n0 count as zero; rhop (or null) multiplies degree n
-// first, dr the factors of a radial derivative.
+// and, with cs not null, the one-degree (ct C, ct S) (leg.cuh), of every
+// family of shs_two.cu that A asks for in the place of C, S (the two-degree
+// pairs of G and J as the differences described there).  Degrees above
+// nmax and S_n0 count as zero; rhop (or null) multiplies degree n first, dr
+// the factors of a radial derivative.
 // Layouts of the degree-ntab tables.  Memory-bound, one pass.  The first
 // `geo` blocks are k_geometry's (which a call without rhop does not have to
 // wait for): one launch and its latency less.
@@ -307,46 +312,87 @@ __global__ void k_two_scale(ScaleArgs A, long long m_lo, GeometryArgs G,
     const long long s0 = tri_col0(A.shc_nmax, m) - m;
     const long long nl = two_len(nmax, m);
     const long long TL = two_sum(A.ntab);
+    const long long T1 = tri_size(A.ntab);
+    // the degree's factor: radius ratio and radial derivative
     auto get = [&](long long n) {
         if (n > nmax)
             return make_double2(0.0, 0.0);
-        const double w = A.rhop ? A.rhop[n] : 1.0;
-        return make_double2(w * A.c[s0 + n], m == 0 ? 0.0 : w * A.s[s0 + n]);
-    };
-    auto amp = [&](long long n) {
-        double w = 1.0;
+        double w = A.rhop ? A.rhop[n] : 1.0;
         if (A.dr >= 1)
             w *= (double)(n + 1);
         if (A.dr >= 2)
             w *= (double)(n + 2);
-        return w;
+        return make_double2(w * A.c[s0 + n], m == 0 ? 0.0 : w * A.s[s0 + n]);
+    };
+    auto times = [](double w, double2 v) {
+        return make_double2(w * v.x, w * v.y);
+    };
+    // member n of family f from the coefficients of degrees n and n + 1
+    auto member = [&](int f, long long n, double2 v, double2 next) {
+        const double nd = (double)n;
+        switch (f)
+        {
+        case 0: return v;
+        case 1: return times(nd, v);
+        case 2: return times(nd * (nd + 1.0), v);
+        default:
+        {
+            // e_n+1: cos(lat) dP_n+1 = e_n+1 P_n - (n + 1) t P_n+1
+            const double q = nd + 1.0, md = (double)m;
+            const double e = sqrt((q - md) * (q + md) * (2.0 * q + 1.0) /
+                                  (2.0 * q - 1.0));
+            return times(f == 3 ? e : e * (q + 1.0), next);
+        }
+        }
     };
     for (long long l = threadIdx.x; l < nl; l += blockDim.x)
     {
         const long long n = m + 2 * l;
-        const double2 e0 = get(n), o = get(n + 1), e1 = get(n + 2);
-        if (A.cs)
+        const double2 v0 = get(n), v1 = get(n + 1), v2 = get(n + 2);
+        const double2 v3 = A.nfam > 1 ? get(n + 3) : v2;
+        const double a1 = A.kw[c0 + l], a2 = A.kw[TL + c0 + l],
+                     a3 = A.kw[2 * TL + c0 + l];
+        for (int i = 0; i < A.nfam; i++)
         {
-            const double k0 = A.tc[t0 + n] * amp(n);
-            A.cs[t0 + n] = make_double2(k0 * e0.x, k0 * e0.y);
-            if (n < nmax)
+            const int f = A.fam[i];
+            const double2 e0 = member(f, n, v0, v1);
+            const double2 o = member(f, n + 1, v1, v2);
+            const double2 e1 = member(f, n + 2, v2, v3);
+            if (A.cs)
             {
-                const double k1 = A.tc[t0 + n + 1] * amp(n + 1);
-                A.cs[t0 + n + 1] = make_double2(k1 * o.x, k1 * o.y);
+                A.cs[i * T1 + t0 + n] = times(A.tc[t0 + n], e0);
+                if (n < nmax)
+                    A.cs[i * T1 + t0 + n + 1] = times(A.tc[t0 + n + 1], o);
             }
+            double2 even = make_double2(fma(a1, e0.x, a2 * e1.x),
+                                        fma(a1, e0.y, a2 * e1.y));
+            double2 odd = times(a3, o);
+            if (f >= 3)
+            {
+                // the differences G - H, J - N in the other parity's place
+                const double2 h0 = member(f - 2, n, v0, v1);
+                const double2 h1 = member(f - 2, n + 1, v1, v2);
+                const double2 h2 = member(f - 2, n + 2, v2, v3);
+                const double2 g = odd;
+                odd = make_double2(g.x - fma(a1, h0.x, a2 * h2.x),
+                                   g.y - fma(a1, h0.y, a2 * h2.y));
+                even = make_double2(even.x - a3 * h1.x, even.y - a3 * h1.y);
+            }
+            double2 *out = A.cs2 + 2 * (i * TL + c0 + l);
+            out[0] = even;
+            out[1] = odd;
         }
-        double a1 = A.kw[c0 + l], a2 = A.kw[TL + c0 + l],
-               a3 = A.kw[2 * TL + c0 + l];
-        if (A.dr > 0)
-        {
-            a1 *= amp(n);
-            a3 *= amp(n + 1);
-            a2 *= amp(n + 2);
-        }
-        A.cs2[2 * (c0 + l)] = make_double2(fma(a1, e0.x, a2 * e1.x),
-                                           fma(a1, e0.y, a2 * e1.y));
-        A.cs2[2 * (c0 + l) + 1] = make_double2(a3 * o.x, a3 * o.y);
     }
+}
+
+void scale_families(ScaleArgs *A, int mode)
+{
+    static const int n[] = {1, 2, 4, 3, 5, 5};
+    static const int f[][5] = {{0},          {3, 1},          {0, 1, 2, 3},
+                               {0, 1, 3},    {0, 1, 2, 3, 4}, {0, 1, 2, 3, 4}};
+    A->nfam = n[mode];
+    for (int i = 0; i < 5; i++)
+        A->fam[i] = f[mode][i];
 }
 
 cudaError_t launch_two_tables(long long nmax, const double *sg, double2 *ab,

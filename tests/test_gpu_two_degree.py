@@ -1,5 +1,5 @@
 """The two-degree recurrence (two.cuh) and the rules that choose it, against
-the CPU oracle: degrees around the rule's lower end, whole and partial
+the CPU oracle: degrees around the rules' lower ends, whole and partial
 32-pair groups, latitudes either side of its equatorial band, every radius
 rule and latitude orders it must leave to the one-degree kernels.
 
@@ -54,7 +54,7 @@ def grids(cb, name, n, r):
 
 
 @pytest.mark.parametrize("name", ["gl", "dh1", "dh2"])
-@pytest.mark.parametrize("nmax", [127, 128, 129, 191, 258])
+@pytest.mark.parametrize("nmax", [191, 399, 400, 401, 447])
 def test_synthesis(cb, name, nmax):
     p, g = grids(cb, name, nmax, R_EARTH)
     f, ref = both(cb, p, g, nmax)
@@ -67,7 +67,7 @@ def test_synthesis(cb, name, nmax):
 @pytest.mark.parametrize("kind", [None, (1, 0, 0), (2, 0, 0), (0, 0, 1),
                                   (0, 0, 2), (1, 0, 1)])
 def test_radii_and_radial_derivatives(cb, ratio, kind):
-    n = 210
+    n = 410
     p, g = grids(cb, "gl", n, R_EARTH * ratio)
     f, ref = both(cb, p, g, n, kind)
     keep = np.repeat(np.abs(p.lat) < np.deg2rad(89.0), p.lon.size)
@@ -79,7 +79,7 @@ def test_radii_and_radial_derivatives(cb, ratio, kind):
 def test_custom_latitudes(cb, case):
     """Orders and spans of latitudes: those that the two-degree kernel takes
     (symmetric, towards the equator) and those that it must not."""
-    n = 160
+    n = 405
     rng = np.random.default_rng(3)
     half = np.sort(rng.uniform(0.003, 1.56, 75))[::-1]
     lat = np.concatenate([half, -half[::-1]])
@@ -122,6 +122,67 @@ def test_columns_that_start_below_the_double_range(cb):
     # next to the pole a rounding of the latitude is a phase n / cos(lat)
     amp = 1.0 / np.cos(lat)
     assert np.all(np.abs(f - ref).max(1) <= tol(n) * amp * rms)
+
+
+# gradients and latitudinal derivatives (families, shs_two.cu) around their
+# smallest degree; the rows next to the poles apart, where a rounding of the
+# latitude alone is 1 / cos(lat)^2 of the result
+@pytest.mark.parametrize("nmax", [127, 128, 163])
+@pytest.mark.parametrize("height", [0.0, 2e5])
+@pytest.mark.parametrize("kind", ["grad1", "grad2", (0, 1, 0), (0, 2, 0),
+                                  (1, 1, 0), (0, 1, 1)])
+def test_latitudinal_derivatives(cb, nmax, height, kind):
+    p, g = grids(cb, "gl", nmax, R_EARTH + height)
+    c, s = model(nmax, 5)
+    shc = cb.Shc(nmax, GM, R_EARTH, c, s)
+    if kind == "grad1":
+        out = cb.shs_point_grad1(p, shc, nmax)
+    elif kind == "grad2":
+        out = cb.shs_point_grad2(p, shc, nmax)
+    else:
+        out = [cb.shs_point_guru(p, shc, nmax, *kind)]
+    ref = orc.shs_point(g, orc.Shc(nmax, GM, R_EARTH, c, s), nmax, kind)
+    u = np.cos(p.lat)
+    for f, o in zip(out, ref):
+        f = np.asarray(f).reshape(p.lat.size, -1)
+        o = np.asarray(o).reshape(p.lat.size, -1)
+        rms = np.sqrt(np.mean(o ** 2))
+        assert np.all(np.sqrt(np.mean((f - o) ** 2, axis=1))
+                      <= 8 * tol(nmax) / u ** 2 * rms)
+        keep = u > 0.2
+        assert rel_rms(f[keep], o[keep]) <= 16 * tol(nmax)
+
+
+def test_batch_equals_single_calls(cb):
+    """All ten quantities in one pass and three single calls form the same
+    sums: the potential, grad1 and grad2 of a set agree bit for bit."""
+    import ctypes as ct
+    import torch
+    from charm_b200._lib import _libcharm as L
+    n = 402
+    p = cb.PointGridGL(n, R_EARTH + 1e4)
+    c, s = kaula(n, 9)
+    d = torch.from_numpy(np.stack([c, s])).cuda()
+    f = torch.empty((10, p.lat.size, p.lon.size), dtype=torch.float64,
+                    device="cuda")
+    P = ct.c_void_p
+    L.charm_b200_shs_point_batch_dev.argtypes = [
+        P, ct.c_size_t, ct.POINTER(ct.c_ulong), ct.POINTER(ct.c_ulong),
+        ct.POINTER(ct.c_double), ct.c_double, ct.POINTER(P), ct.POINTER(P),
+        ct.c_int, ct.POINTER(P), P]
+    nm, mu = (ct.c_ulong * 1)(n), (ct.c_double * 1)(GM)
+    err = L.charm_err_init()
+    L.charm_b200_shs_point_batch_dev(
+        ct.cast(p._Point, P), 1, nm, nm, mu, R_EARTH,
+        (P * 1)(d[0].data_ptr()), (P * 1)(d[1].data_ptr()), 3,
+        (P * 1)(f.data_ptr()), ct.cast(err, P))
+    assert L.charm_err_isempty(err)
+    L.charm_err_free(err)
+    shc = cb.Shc(n, GM, R_EARTH, c, s)
+    one = ([cb.shs_point(p, shc, n)] + list(cb.shs_point_grad1(p, shc, n))
+           + list(cb.shs_point_grad2(p, shc, n)))
+    for q in range(10):
+        assert np.array_equal(f[q].cpu().numpy(), np.asarray(one[q])), q
 
 
 # either side of the rule's smallest grid (384 pairs, degree 512), whole and
