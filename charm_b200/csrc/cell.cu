@@ -256,9 +256,13 @@ __device__ __forceinline__ void lon_factors(long long m, double dlon,
 // q_m = (t2 P_mm(t2) - t1 P_mm(t1)) / (m + 1) from the sectorial seeds of
 // leg.cuh (P_mm = S_m u^m, S_m = sqrt(3) prod d_k, src/leg/
 // leg_func_prepare.c; below the double range it is zero, as CHarm's
-// X-numbers convert).  k_cell_imm_rec: one thread per pair runs the
-// recurrence over the orders, I_mm = g_m I_m-2,m-2 + q_m, from the closed
-// forms of I_11 and I_22, in place.  imm is order-major ([m][pair]), so
+// X-numbers convert).  k_cell_imm_rec runs the recurrence over
+// the orders, I_mm = g_m I_m-2,m-2 + q_m, from the closed forms of I_11 and
+// I_22, in place: a block of 32 pairs, one per lane, whose warps take
+// consecutive stretches of orders, first from zero (with the product of the
+// stretch's g_m), then, the stretches before it combined, from its true start.
+// Bound by the latency of its loads: one thread per pair walking all orders
+// took 96 us at nmax 719, this takes 11.  imm is order-major ([m][pair]), so
 // that the writes and the reads by the warps of one order are coalesced.
 __global__ void k_cell_imm_q(CellArgs A)
 {
@@ -280,12 +284,16 @@ __global__ void k_cell_imm_q(CellArgs A)
     A.imm[(size_t)m * np + p] = A.hn[m].y * (t2 * p2 - t1 * p1);
 }
 
-__global__ void k_cell_imm_rec(CellArgs A)
+constexpr int IMM_WARPS = 32;
+
+__global__ void __launch_bounds__(IMM_WARPS * 32) k_cell_imm_rec(CellArgs A)
 {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    __shared__ double sb[2][IMM_WARPS][32];
+    __shared__ double sa[2][IMM_WARPS];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int np = A.npairs;
-    if (p >= np)
-        return;
+    const bool valid = (int)blockIdx.x * 32 + lane < np;
+    const int p = valid ? blockIdx.x * 32 + lane : np - 1;
     const long long N = A.nmax;
     const double ROOT3 = 1.73205080756887729353;
     const double PI_2 = 1.57079632679489661923;
@@ -293,39 +301,65 @@ __global__ void k_cell_imm_rec(CellArgs A)
     const double t2 = A.geo[2 * np + p], u2 = A.geo[3 * np + p];
     const double la1 = A.geo[6 * np + p], la2 = A.geo[7 * np + p];
     double *io = A.imm + p;
-    io[0] = 0.0;
     // the closed forms of CHarm (shs_cell_kernel.c:229-262)
-    double im2 = (ROOT3 / 2.0) * ((t2 * u2 - (PI_2 - la2)) -
-                                  (t1 * u1 - (PI_2 - la1)));
-    io[(size_t)np] = im2;
-    if (N < 2)
-        return;
-    double im1 = (3.87298334620741688518 / 6.0) *
-                 (t2 * (3.0 - t2 * t2) - t1 * (3.0 - t1 * t1));
-    io[2 * (size_t)np] = im1;
-    constexpr int B = 8;
-    for (long long m0 = 3; m0 <= N; m0 += B)
+    double v0 = (ROOT3 / 2.0) * ((t2 * u2 - (PI_2 - la2)) -
+                                 (t1 * u1 - (PI_2 - la1)));
+    double v1 = (3.87298334620741688518 / 6.0) *
+                (t2 * (3.0 - t2 * t2) - t1 * (3.0 - t1 * t1));
+    if (w == 0 && valid)
     {
-        double q[B], gv[B];
-#pragma unroll
-        for (int b = 0; b < B; b++)
-        {
-            const long long m = m0 + b;
-            q[b] = m <= N ? io[(size_t)m * np] : 0.0;
-            gv[b] = m <= N ? __ldg(&A.gm[m]) : 0.0;
-        }
-#pragma unroll
-        for (int b = 0; b < B; b++)
-        {
-            const long long m = m0 + b;
-            if (m > N)
-                break;
-            const double v = fma(gv[b], im2, q[b]);
-            io[(size_t)m * np] = v;
-            im2 = im1;
-            im1 = v;
-        }
+        io[0] = 0.0;
+        io[(size_t)np] = v0;
+        if (N >= 2)
+            io[2 * (size_t)np] = v1;
     }
+    // this warp's orders: an even number, so that the two parities' chains
+    // (from v0 and v1) keep their places
+    const long long len =
+        N > 2 ? 2 * ((N - 2 + 2 * IMM_WARPS - 1) / (2 * IMM_WARPS)) : 0;
+    const long long m0 = 3 + w * len;
+    const long long m1 = m0 + len < N + 1 ? m0 + len : N + 1;
+    constexpr int B = 8;
+    // both walks over the orders: step(m, q_m, g_m, chain)
+    auto walk = [&](auto step) {
+        for (long long m = m0; m < m1; m += B)
+        {
+            double q[B], g[B];
+#pragma unroll
+            for (int b = 0; b < B; b++)
+            {
+                q[b] = m + b < m1 ? io[(size_t)(m + b) * np] : 0.0;
+                g[b] = m + b < m1 ? __ldg(&A.gm[m + b]) : 1.0;
+            }
+#pragma unroll
+            for (int b = 0; b < B; b++)
+                step(m + b, q[b], g[b], b & 1);
+        }
+    };
+    double a[2] = {1.0, 1.0}, s[2] = {0.0, 0.0};
+    walk([&](long long, double q, double g, int c) {
+        s[c] = fma(g, s[c], q);
+        a[c] *= g;
+    });
+    sb[0][w][lane] = s[0];
+    sb[1][w][lane] = s[1];
+    if (lane == 0)
+    {
+        sa[0][w] = a[0];
+        sa[1][w] = a[1];
+    }
+    __syncthreads();
+    for (int k = 0; k < w; k++)
+    {
+        v0 = fma(sa[0][k], v0, sb[0][k][lane]);
+        v1 = fma(sa[1][k], v1, sb[1][k][lane]);
+    }
+    double v[2] = {v0, v1};
+    walk([&](long long m, double q, double g, int c) {
+        v[c] = fma(g, v[c], q);
+        if (m < m1 && valid)
+            io[(size_t)m * np] = v[c];
+    });
 }
 
 // ---------------------------------------------------------------------------
@@ -1273,9 +1307,7 @@ cudaError_t launch_cell_imm(const CellArgs &A, cudaStream_t st)
         return cudaSuccess;
     const long long total = A.nmax * (long long)A.npairs;
     k_cell_imm_q<<<(unsigned)((total + 255) / 256), 256, 0, st>>>(A);
-    const int threads = 32;
-    k_cell_imm_rec<<<(A.npairs + threads - 1) / threads, threads, 0, st>>>(
-        A);
+    k_cell_imm_rec<<<(A.npairs + 31) / 32, IMM_WARPS * 32, 0, st>>>(A);
     return cudaGetLastError();
 }
 
