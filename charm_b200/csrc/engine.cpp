@@ -2208,7 +2208,9 @@ Status shs_sctr(Context &c, const charm_point *pnt, const CoefIn &in,
     unsigned *d_status;
     unsigned long long *d_counter;
     CB_TRY(status_words(c, &d_status, &d_counter));
-    const int K = choose_k(kgrad, dlat, (long long)npt);
+    // (few points: narrow tiles, so that the items still fill the GPU)
+    const int K = std::min(choose_k(kgrad, dlat, (long long)npt),
+                           npt >= 16384 ? 4 : (npt >= 4096 ? 2 : 1));
     SctrArgs A{};
     A.nmax = (long long)nmax;
     A.npoint = (long long)npt;
@@ -2229,7 +2231,31 @@ Status shs_sctr(Context &c, const charm_point *pnt, const CoefIn &in,
     A.polar_thr = polar_threshold(nmax);
     A.counter = d_counter;
     A.status = d_status;
-    int grid = (int)std::min<long long>((A.ntiles + 3) / 4,
+    // few tiles: each cut into ranges of orders of about equal numbers of
+    // coefficients, enough for four items per resident warp, none below 512
+    // coefficients (an item's own cost is that of some hundred)
+    const long long T = (long long)(nmax + 1) * (nmax + 2) / 2;
+    const long long want = 4LL * 16 * c.num_sms;
+    A.nsplit = (int)std::max<long long>(
+        1, std::min<long long>({(want + A.ntiles - 1) / A.ntiles, T / 512,
+                                64}));
+    std::vector<long long> mb{0};
+    if (A.nsplit > 1)
+    {
+        for (long long m = 1; m <= (long long)nmax; m++)
+            if ((int)mb.size() < A.nsplit &&
+                tri_start((long long)nmax, m) >=
+                    (long long)mb.size() * T / A.nsplit)
+                mb.push_back(m);
+        A.nsplit = (int)mb.size();
+        mb.push_back((long long)nmax + 1);
+        long long *dmb = nullptr;
+        CB_TRY(dbuf(c, "sctr_mb", mb.size(), &dmb));
+        CB_TRY(h2d_small(c, dmb, mb.data(), mb.size() * sizeof(long long)));
+        A.mb = dmb;
+        CB_TRY(dbuf(c, "sctr_part", (size_t)A.nsplit * npar * npt, &A.part));
+    }
+    int grid = (int)std::min<long long>((A.ntiles * A.nsplit + 3) / 4,
                                         (long long)c.num_sms * 8);
     {
         Scope sc(c, TIMER_SCTR);

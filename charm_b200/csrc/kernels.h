@@ -298,6 +298,11 @@ struct SctrArgs
     double mur;
     int dlon;
     double polar_thr;
+    // ranges of orders [mb[k], mb[k + 1]) (device), whose sums go to
+    // part[k][npar][npoint]; nsplit 1: all orders, straight to f
+    int nsplit;
+    const long long *mb;
+    double *part;
     unsigned long long *counter;
     unsigned *status;
 };
