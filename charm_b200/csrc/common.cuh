@@ -100,7 +100,9 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t *bar,
     for (unsigned it = 0; it < limit; ++it)
         if (mbar_try_wait(bar, parity))
             return true;
-    atomicOr(status, DEV_ERR_WAIT_TIMEOUT);
+    // (no atomic: the word may lie in the host's memory)
+    volatile unsigned *const s = status;
+    *s = *s | DEV_ERR_WAIT_TIMEOUT;
     return false;
 }
 

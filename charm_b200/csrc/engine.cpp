@@ -82,6 +82,7 @@ constexpr int SHS_LAT_BANDS = 4;   // synthesis: grid rows down
 constexpr int SHA_LAT_BANDS = 4;   // analysis: grid rows up
 constexpr int SHS_ORD_BANDS = 4;   // synthesis: coefficients up
 constexpr int SHA_ORD_BANDS = 4;   // analysis: coefficients down
+constexpr size_t DEFER_SLOTS = 64;
 constexpr int EV_LAT0 = 0, EV_ORD0 = 6, EV_START = 15;
 
 struct Context
@@ -98,8 +99,15 @@ struct Context
     // orders, EV_START the start of the copy stream after the work already
     // on the compute stream
     cudaEvent_t band_ev[16] = {};
-    // page-locked copy of the device status word read at the end of a call
+    // page-locked status word: the grid calls' kernels write it directly, the
+    // others' device word is copied here at the end of a call
     unsigned *h_status = nullptr;
+    // a sequence of grid calls whose synchronisations wait for its end
+    // (gfm_global_impl): each call stages its uploads in a page-locked slot
+    // of its own, DEFER_SLOTS of them before the sequence must wait
+    bool deferred = false;
+    std::vector<std::pair<void *, size_t>> defer_pins;
+    size_t defer_k = 0;
     std::map<std::string, DevBuf> bufs;
     void *pinned = nullptr;
     size_t pinned_bytes = 0;
@@ -346,6 +354,31 @@ Status pinned(Context &c, size_t bytes, void **out)
         CB_CUDA(cudaMallocHost(&p, std::max<size_t>(bytes, 16)), st);
         c.capture_pins.push_back(p);
         *out = p;
+        return st;
+    }
+    if (c.deferred)
+    {
+        if (c.defer_k == DEFER_SLOTS)
+        {
+            CB_CUDA(cudaStreamSynchronize(c.stream), st);
+            c.defer_k = 0;
+        }
+        if (c.defer_pins.size() <= c.defer_k)
+            c.defer_pins.emplace_back(nullptr, 0);
+        auto &s = c.defer_pins[c.defer_k++];
+        if (s.second < bytes)
+        {
+            if (s.first)
+            {
+                cudaStreamSynchronize(c.stream);
+                cudaFreeHost(s.first);
+                s = {nullptr, 0};
+            }
+            const size_t want = std::max<size_t>(bytes, 1 << 16);
+            CB_CUDA(cudaMallocHost(&s.first, want), st);
+            s.second = want;
+        }
+        *out = s.first;
         return st;
     }
     if (c.pinned_bytes < bytes)
@@ -1358,13 +1391,18 @@ Status finish(Context &c, unsigned *d_status)
     Status st;
     if (c.capturing)
         return st;   // read by batch_graph_launch after each replay
-    // into page-locked memory, so the copy is queued like a kernel and the
-    // one synchronisation below covers both
-    *c.h_status = 0u;
-    CB_CUDA(cudaMemcpyAsync(c.h_status, d_status, sizeof(unsigned),
-                            cudaMemcpyDeviceToHost, c.stream), st);
+    if (c.deferred)
+        return st;   // at the end of the sequence
+    if (d_status != c.h_status)
+    {
+        // into page-locked memory, so the copy is queued like a kernel and
+        // the one synchronisation below covers both
+        *c.h_status = 0u;
+        CB_CUDA(cudaMemcpyAsync(c.h_status, d_status, sizeof(unsigned),
+                                cudaMemcpyDeviceToHost, c.stream), st);
+    }
     CB_CUDA(cudaStreamSynchronize(c.stream), st);
-    const unsigned h_status = *c.h_status;
+    const unsigned h_status = *static_cast<volatile unsigned *>(c.h_status);
     if (c.timing)
         resolve_timers(c);
     if (h_status)
@@ -1613,10 +1651,6 @@ Status grid_geometry(Context &c, const charm_point *pnt, const Pairs &P,
         sincos(hlat[p], &ht[p], &hu[p]);
     void *dgeo = nullptr;
     CB_TRY(buf(c, "geo", up + (size_t)np * 3 * 8, &dgeo));
-    CB_CUDA(cudaMemcpyAsync(dgeo, hp,
-                            up + (plain || G->npole > 0 ? (size_t)np * 2 * 8
-                                                        : 0),
-                            cudaMemcpyHostToDevice, c.stream), st);
     double *d = static_cast<double *>(dgeo);
     G->lat = d;
     G->rhos = G->w_n = d + np;
@@ -1629,19 +1663,24 @@ Status grid_geometry(Context &c, const charm_point *pnt, const Pairs &P,
     G->z = dt + 2 * np;
     void *sp = nullptr;
     CB_TRY(buf(c, "status", 256, &sp));
-    G->d_status = static_cast<unsigned *>(sp);
+    // the status word is written to page-locked memory (in a captured graph
+    // to device memory, cleared by the graph itself)
+    G->d_status = c.capturing ? static_cast<unsigned *>(sp) : c.h_status;
+    if (!c.capturing && !c.deferred)
+        *c.h_status = 0u;
     G->counter = reinterpret_cast<unsigned long long *>(
         static_cast<char *>(sp) + 64);
-    if (plain)
-    {
-        CB_CUDA(cudaMemsetAsync(sp, 0, 256, c.stream), st);
-        return st;
-    }
     GeometryArgs A{};
+    // k_geometry reads the page-locked staging itself and leaves the copy
+    // the other kernels read
+    A.src = hlat;
+    A.dst = d;
+    A.words = (plain ? 6 : 4) * (long long)np;
+    A.plain = plain ? 1 : 0;
     A.npairs = np;
     A.polar = G->polar;
     A.given = G->npole;
-    A.lat = d;
+    A.lat = hlat;
     A.t = dt;
     A.u = dt + np;
     A.z = dt + 2 * np;
@@ -1653,7 +1692,7 @@ Status grid_geometry(Context &c, const charm_point *pnt, const Pairs &P,
         A.pw = pw;
         G->pw = pw;
     }
-    A.clear = G->d_status;
+    A.clear = static_cast<unsigned *>(sp);
     if (G->rho != 1.0)
     {
         CB_TRY(dbuf(c, "geo_rhop", (size_t)(nmax + 1), &G->rhop));
@@ -1855,9 +1894,9 @@ Status shs_grid(Context &c, const charm_point *pnt, const CoefIn &in,
         S.dr = kgrad == 0 ? dr : 0;
         S.cs = dcs;
         S.cs2 = dcs2;
-        const bool with = G.pending && dcs2 && m_hi > m_lo;
-        CB_CUDA(launch_scale_orders(S, m_lo, m_hi, c.stream,
-                                    with ? &G.args : nullptr), s2);
+        const bool with = G.pending && m_hi > m_lo;
+        CB_CUDA(launch_two_scale(S, m_lo, m_hi, with ? &G.args : nullptr,
+                                 c.stream), s2);
         if (with)
             G.pending = false;
         return s2;
@@ -2474,10 +2513,10 @@ Status shs_batch(Context &c, const charm_point *pnt, size_t nsets,
         S.rhop = G.rhop;
         S.cs = cs_all ? cs_all + (size_t)j * T : nullptr;
         S.cs2 = cs2_all ? cs2_all + (size_t)j * T2 : nullptr;
-        const bool with = G.pending && S.cs2;
+        const bool with = G.pending;
         Scope sc(c, TIMER_PREP);
-        CB_CUDA(launch_scale_orders(S, 0, S.nmax + 1, c.stream,
-                                    with ? &G.args : nullptr), st);
+        CB_CUDA(launch_two_scale(S, 0, S.nmax + 1, with ? &G.args : nullptr,
+                                 c.stream), st);
         if (with)
             G.pending = false;
     }
@@ -2708,7 +2747,7 @@ Status shs_batch(Context &c, const charm_point *pnt, size_t nsets,
             // the set descriptors and the lumped buffer are reused by the
             // next sub-batch: wait for this one (stream order suffices
             // inside a captured graph, whose uploads have their own copies)
-            if (!c.capturing)
+            if (!c.capturing && !c.deferred)
                 CB_CUDA(cudaStreamSynchronize(c.stream), st);
         }
     }
@@ -4662,6 +4701,26 @@ Status gfm_global_impl(Context &c, const GfmArgs &g)
                             c.stream), st);
     // (a pageable source: the copy has read vh when the call returns)
 
+    // One synchronisation at the end instead of one per transform (the
+    // partial exports copy and check in between, so they keep them)
+    struct Deferred
+    {
+        Context &c;
+        bool on;
+        ~Deferred()
+        {
+            if (on)
+                cudaStreamSynchronize(c.stream);
+            c.deferred = false;
+        }
+    } defer{c, !g.hro_path && !g.pot_path};
+    if (defer.on)
+    {
+        *c.h_status = 0u;
+        c.deferred = true;
+        c.defer_k = 0;
+    }
+
     // The shape and the densities of one power share its grid: one batched
     // synthesis forms all of them (sets of their own degrees, one launch)
     // when their grids and lumped coefficients (about as large again) fit
@@ -4769,6 +4828,15 @@ Status gfm_global_impl(Context &c, const GfmArgs &g)
         CB_TRY(download_tri(c, dpot, np, g.pot->c));
         CB_TRY(download_tri(c, dpot + Tp, np, g.pot->s));
         CB_CUDA(cudaStreamSynchronize(c.stream), st);
+    }
+    if (defer.on)
+    {
+        c.deferred = false;
+        defer.on = false;
+        CB_TRY(finish(c, c.h_status));
+    }
+    if (g.pot)
+    {
         g.pot->mu = gm;
         g.pot->r = g.R;
     }
@@ -5787,6 +5855,9 @@ void shutdown()
     if (c.h_status)
         cudaFreeHost(c.h_status);
     c.h_status = nullptr;
+    for (auto &s : c.defer_pins)
+        cudaFreeHost(s.first);
+    c.defer_pins.clear();
     for (int b = 0; b < RING_N; b++)
     {
         if (c.ring[b])

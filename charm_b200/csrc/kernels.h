@@ -115,9 +115,15 @@ struct ShsTwoArgs
 constexpr int GEO_CLEAR_WORDS = 64;
 struct GeometryArgs
 {
+    // page-locked staging of the call, copied to dst (8-byte words)
+    const double *src;
+    double *dst;
+    long long words;
+    int plain;             // 1: nothing but that copy and `clear`
     int npairs;
     int polar;             // pairs below this store z = -cos^2, else sin^2
-    int given;             // pairs below this have t and u already
+    int given;             // pairs below this take t and u from src (behind
+                           // the words that are copied)
     const double *lat;
     double *t, *u, *z;
     double2 *pw;           // power table of two_seed, npow entries (or 0)
@@ -424,11 +430,6 @@ cudaError_t launch_tables(long long nmax, const double *r, const double *ri,
                           const double *smm, double2 *tb, double *tc,
                           double *tmul, int ldmul, double *sg,
                           cudaStream_t st);
-// k_scale_cs for the orders [m_lo, m_hi) only
-// orders [m_lo, m_hi) in the forms A asks for
-cudaError_t launch_scale_orders(const ScaleArgs &A, long long m_lo,
-                                long long m_hi, cudaStream_t st,
-                                const GeometryArgs *G = nullptr);
 cudaError_t launch_scale_cs(long long nmax, long long shc_nmax,
                             const double *c, const double *s,
                             const double *tc, double2 *cs, cudaStream_t st);
@@ -462,9 +463,9 @@ cudaError_t launch_two_tables(long long nmax, const double *sg, double2 *ab,
                               double2 *ag, double *kw, double *sm,
                               cudaStream_t st);
 cudaError_t launch_geometry(const GeometryArgs &G, cudaStream_t st);
-// orders [m_lo, m_hi); A.cs2 must not be null
-// (G not null: the blocks of launch_geometry in the same launch; G->rhop
-// must be null)
+// the coefficients of the orders [m_lo, m_hi) in the forms A asks for (G not
+// null: the blocks of launch_geometry in the same launch; G->rhop must be
+// null)
 cudaError_t launch_two_scale(const ScaleArgs &A, long long m_lo,
                              long long m_hi, const GeometryArgs *G,
                              cudaStream_t st);

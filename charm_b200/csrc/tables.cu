@@ -121,32 +121,24 @@ __global__ void k_tables(long long nmax, const double *__restrict__ r,
     sg[2 * m + 1] = (double)g0;
 }
 
-// (ct C_nm, ct S_nm) up to degree nmax, in the layout of the degree-ntab
-// tables, from the caller's C, S triangles of degree shc_nmax, times rhop[n] when not null; S_n0 forced to
-// zero (CHarm never reads it, src/shs/shs_point_kernel.c:1014-1248).
-__global__ void k_scale_cs(long long ntab, long long nmax,
-                           long long shc_nmax,
+// (ct C_nm, ct S_nm) of the degree-nmax triangle from the caller's C, S
+// triangles of degree shc_nmax; S_n0 forced to zero (CHarm never reads it,
+// src/shs/shs_point_kernel.c:1014-1248).
+__global__ void k_scale_cs(long long nmax, long long shc_nmax,
                            const double *__restrict__ c,
                            const double *__restrict__ s,
-                           const double *__restrict__ tc,
-                           const double *__restrict__ rhop, double2 *cs,
-                           long long m_lo)
+                           const double *__restrict__ tc, double2 *cs)
 {
-    long long m = m_lo + blockIdx.x;
+    long long m = blockIdx.x;
     if (m > nmax)
         return;
-    long long c0 = tri_col0(ntab, m);
+    long long c0 = tri_col0(nmax, m);
     long long s0 = tri_col0(shc_nmax, m);
     for (long long n = m + threadIdx.x; n <= nmax; n += blockDim.x)
     {
         double k = tc[c0 + n - m];
-        double vc = c[s0 + n - m], vs = m == 0 ? 0.0 : s[s0 + n - m];
-        if (rhop)
-        {
-            vc *= rhop[n];
-            vs *= rhop[n];
-        }
-        cs[c0 + n - m] = make_double2(k * vc, k * vs);
+        cs[c0 + n - m] = make_double2(k * c[s0 + n - m],
+                                      m == 0 ? 0.0 : k * s[s0 + n - m]);
     }
 }
 
@@ -206,21 +198,7 @@ cudaError_t launch_scale_cs(long long nmax, long long shc_nmax,
                             const double *c, const double *s,
                             const double *tc, double2 *cs, cudaStream_t st)
 {
-    k_scale_cs<<<(int)(nmax + 1), 128, 0, st>>>(nmax, nmax, shc_nmax, c, s,
-                                                tc, nullptr, cs, 0);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_scale_orders(const ScaleArgs &A, long long m_lo,
-                                long long m_hi, cudaStream_t st,
-                                const GeometryArgs *G)
-{
-    if (m_hi <= m_lo)
-        return cudaSuccess;
-    if (A.cs2)
-        return launch_two_scale(A, m_lo, m_hi, G, st);
-    k_scale_cs<<<(int)(m_hi - m_lo), 128, 0, st>>>(
-        A.ntab, A.nmax, A.shc_nmax, A.c, A.s, A.tc, A.rhop, A.cs, m_lo);
+    k_scale_cs<<<(int)(nmax + 1), 128, 0, st>>>(nmax, shc_nmax, c, s, tc, cs);
     return cudaGetLastError();
 }
 

@@ -134,8 +134,9 @@ __global__ void k_two_tables(long long nmax, const double *sg, double2 *ab,
 // Latitudes.  Per pair, from the double-double sine and cosine of its
 // latitude (Taylor series of lat / 8, doubled three times): t, u rounded;
 // z = x2, or -u2 for the pairs below `polar`; and (by > 0) the power
-// table of two_seed, POW_STRETCH entries per thread.  The first block also
-// clears the status and counter words of the call and fills the powers
+// table of two_seed, POW_STRETCH entries per thread.  The first row of blocks
+// also copies the call's page-locked staging to the device (one launch in the
+// place of a copy and a memset), clears its counters and fills the powers
 // rhop[n] = rho^n, n = 0..nmax, of the one radius ratio rho (1 + drho)
 // of the call (drho: its relative rounding error).  Latency-bound: chains
 // of some hundred dependent operations whatever the sizes (with the series
@@ -149,7 +150,10 @@ constexpr int GEO_THREADS = 128;
 
 __host__ __device__ __forceinline__ int geo_blocks_x(const GeometryArgs &G)
 {
-    return G.npairs > 0 ? (G.npairs + GEO_THREADS - 1) / GEO_THREADS : 1;
+    // a thread per pair, and per 16 bytes of the staging: each of its reads
+    // takes more than a microsecond, so none waits for another
+    const long long n = G.words / 2 > G.npairs ? G.words / 2 : G.npairs;
+    return n > 0 ? (int)((n + GEO_THREADS - 1) / GEO_THREADS) : 1;
 }
 
 __host__ __device__ __forceinline__ int geo_blocks_y(const GeometryArgs &G)
@@ -201,6 +205,10 @@ __device__ void geometry_block(const GeometryArgs &G, int bx, int by)
     {
         if (bx == 0 && threadIdx.x < GEO_CLEAR_WORDS)
             G.clear[threadIdx.x] = 0u;
+        // (an even number of words)
+        if (2LL * p < G.words)
+            reinterpret_cast<double2 *>(G.dst)[p] =
+                reinterpret_cast<const double2 *>(G.src)[p];
         if (G.rhop)
             for (long long n = p; n <= G.nmax;
                  n += (long long)geo_blocks_x(G) * GEO_THREADS)
@@ -210,7 +218,7 @@ __device__ void geometry_block(const GeometryArgs &G, int bx, int by)
                 G.rhop[n] = scalbn(v.v.hi, v.e);
             }
     }
-    if (p >= G.npairs)
+    if (p >= G.npairs || G.plain)
         return;
     // sin h / h and cos h at h = lat / 8 (h^2 < 0.04): the terms from h^6 on
     // in double (below 2^-26, so good to 2^-79), the first two in
@@ -249,11 +257,9 @@ __device__ void geometry_block(const GeometryArgs &G, int bx, int by)
     }
     if (by == 0)
     {
-        if (p >= G.given)
-        {
-            G.t[p] = s.hi;
-            G.u[p] = c.hi;
-        }
+        const bool given = p < G.given;
+        G.t[p] = given ? G.src[4 * (long long)G.npairs + p] : s.hi;
+        G.u[p] = given ? G.src[5 * (long long)G.npairs + p] : c.hi;
         G.z[p] = p < G.polar ? -dd_mul(c, c).hi : dd_mul(s, s).hi;
         return;
     }
@@ -309,6 +315,23 @@ __global__ void k_two_scale(ScaleArgs A, long long m_lo, GeometryArgs G,
         return;
     const long long c0 = two_col0(A.ntab, m);
     const long long t0 = tri_col0(A.ntab, m) - m;
+    if (!A.cs2)
+    {
+        // the one-degree form of C, S alone
+        const long long s1 = tri_col0(A.shc_nmax, m) - m;
+        for (long long n = m + threadIdx.x; n <= nmax; n += blockDim.x)
+        {
+            double k = A.tc[t0 + n];
+            double vc = A.c[s1 + n], vs = m == 0 ? 0.0 : A.s[s1 + n];
+            if (A.rhop)
+            {
+                vc *= A.rhop[n];
+                vs *= A.rhop[n];
+            }
+            A.cs[t0 + n] = make_double2(k * vc, k * vs);
+        }
+        return;
+    }
     const long long s0 = tri_col0(A.shc_nmax, m) - m;
     const long long nl = two_len(nmax, m);
     const long long TL = two_sum(A.ntab);
