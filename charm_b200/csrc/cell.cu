@@ -114,6 +114,70 @@ __device__ __forceinline__ void stage_chunk(const Stage &S, const CellArgs &A,
     __syncwarp();
 }
 
+// Stages chunk j of the zonal column: entry i of degree n = 64 j + i holds
+// the factors of P_n+1 in tb and, in hn.x, that of the integral over ct_n
+// (1 / ct_n at n = 0, whose integral is t2 - t1).  The items of order 0 are
+// the longest chain of a launch: with the table loads and the division by
+// ct_n in their loop over the degrees, they alone kept the kernels of nmax
+// 719 (361 pairs of rows) at 249 us of synthesis and 265 us of analysis; with
+// the stage these take 117 and 181.
+__device__ __forceinline__ void stage_zonal(const Stage &S, const CellArgs &A,
+                                            int j, int cnt, unsigned lane)
+{
+    __syncwarp();
+    const long long off = (long long)j * LEG_CHUNK;
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+    {
+        const int i = (int)lane + 32 * h;
+        if (i < cnt)
+        {
+            const long long n = off + i;
+            double4 z = make_double4(0.0, 0.0, 1.0, 0.0);
+            if (n > 0)
+                z = A.zn[n];
+            const double ct = A.tc[n];
+            if (S.cs)
+                S.cs[i] = A.cs[n];
+            S.tb[i] = make_double2(z.x, z.y);
+            S.hn[i] = make_double2(z.z / ct, 0.0);
+        }
+    }
+    __syncwarp();
+}
+
+// The zonal polynomials of one cell row at its two boundaries (p1: P_n,
+// p0: P_n-1): returns I_n0 / ct_n of degree n from the staged factors
+struct ZonalRec
+{
+    double t1, t2, p0a, p0b, p1a, p1b;
+
+    __device__ __forceinline__ void seed(double ta, double tb)
+    {
+        t1 = ta;
+        t2 = tb;
+        p0a = p0b = 1.0;
+        p1a = ta;
+        p1b = tb;
+    }
+
+    __device__ __forceinline__ double step(const Stage &S, int i, bool first)
+    {
+        const double w = S.hn[i].x;
+        if (first)
+            return (t2 - t1) * w;
+        const double2 z = S.tb[i];
+        const double p2a = z.x * (t1 * p1a) - z.y * p0a;
+        const double p2b = z.x * (t2 * p1b) - z.y * p0b;
+        const double v = w * ((p2b - p0b) - (p2a - p0a));
+        p0a = p1a;
+        p1a = p2a;
+        p0b = p1b;
+        p1b = p2b;
+        return v;
+    }
+};
+
 // The two boundary recurrences and the integral of one cell row: state
 // (x, y, E) per boundary as in leg.cuh, (J0, J1) = (J~_n-2, J~_n-1), and
 // the weights w = u^2 of the boundaries that are in the double range.
@@ -411,30 +475,17 @@ __global__ void __launch_bounds__(CELL_WARPS * 32) k_shs_cell(CellArgs A)
         {
             // zonal: un-normalised polynomials (shs_cell_kernel.c:97-175);
             // the sums take I_n0 / ct_n against ct_n C_n0
-            double p0a = 1.0, p0b = 1.0, p1a = R.t1, p1b = R.t2;
+            ZonalRec Z;
+            Z.seed(R.t1, R.t2);
             for (int j = 0; j < nchunks; j++)
             {
                 const int cnt = (int)min((long long)LEG_CHUNK,
                                          ncol - (long long)j * LEG_CHUNK);
-                stage_chunk(S, A, c0, m, j, cnt, lane);
+                stage_zonal(S, A, j, cnt, lane);
                 for (int i = 0; i < cnt; i++)
                 {
                     const long long n = (long long)j * LEG_CHUNK + i;
-                    double in0;
-                    if (n == 0)
-                        in0 = R.t2 - R.t1;
-                    else
-                    {
-                        const double4 z = A.zn[n];
-                        const double p2a = z.x * (R.t1 * p1a) - z.y * p0a;
-                        const double p2b = z.x * (R.t2 * p1b) - z.y * p0b;
-                        in0 = z.z * ((p2b - p0b) - (p2a - p0a));
-                        p0a = p1a;
-                        p1a = p2a;
-                        p0b = p1b;
-                        p1b = p2b;
-                    }
-                    const double v = (in0 / A.tc[c0 + n]) * rn;
+                    const double v = Z.step(S, i, n == 0) * rn;
                     if (RR)
                         rn *= rho;
                     const double2 c = S.cs[i];
@@ -601,38 +652,22 @@ __global__ void __launch_bounds__(CELL_WARPS * 32) k_shs_cell2(CellArgs A)
         {
             // zonal: un-normalised polynomials (shs_cell_kernel.c:97-175),
             // row by row
-            double p0a[2] = {1.0, 1.0}, p0b[2] = {1.0, 1.0};
-            double p1a[2] = {R[0].t1, R[1].t1}, p1b[2] = {R[0].t2, R[1].t2};
+            ZonalRec Z[2];
+            Z[0].seed(R[0].t1, R[0].t2);
+            Z[1].seed(R[1].t1, R[1].t2);
             for (int j = 0; j < nchunks; j++)
             {
                 const int cnt = (int)min((long long)LEG_CHUNK,
                                          ncol - (long long)j * LEG_CHUNK);
-                stage_chunk(S, A, c0, m, j, cnt, lane);
+                stage_zonal(S, A, j, cnt, lane);
                 for (int i = 0; i < cnt; i++)
                 {
                     const long long n = (long long)j * LEG_CHUNK + i;
-                    const double tcn = A.tc[c0 + n];
                     const double2 c = S.cs[i];
 #pragma unroll
                     for (int k = 0; k < 2; k++)
                     {
-                        double in0;
-                        if (n == 0)
-                            in0 = R[k].t2 - R[k].t1;
-                        else
-                        {
-                            const double4 z = A.zn[n];
-                            const double p2a =
-                                z.x * (R[k].t1 * p1a[k]) - z.y * p0a[k];
-                            const double p2b =
-                                z.x * (R[k].t2 * p1b[k]) - z.y * p0b[k];
-                            in0 = z.z * ((p2b - p0b[k]) - (p2a - p0a[k]));
-                            p0a[k] = p1a[k];
-                            p1a[k] = p2a;
-                            p0b[k] = p1b[k];
-                            p1b[k] = p2b;
-                        }
-                        const double v = (in0 / tcn) * rn[k];
+                        const double v = Z[k].step(S, i, n == 0) * rn[k];
                         if (RR)
                             rn[k] *= rho[k];
                         if ((n & 1) == 0)
@@ -814,7 +849,6 @@ __global__ void __launch_bounds__(CELL_WARPS * 32, K == 1 ? 3 : 2)
         {
             CellRec R[K];
             double amp[K], amm[K], bmp[K], bmm[K];
-            double p0a[K], p0b[K], p1a[K], p1b[K];
             bool all_skip = true, any_scaled = false;
 #pragma unroll
             for (int k = 0; k < K; k++)
@@ -863,9 +897,6 @@ __global__ void __launch_bounds__(CELL_WARPS * 32, K == 1 ? 3 : 2)
                         bmm[k] = bm * sm - am * cm;
                     }
                 }
-                p0a[k] = p0b[k] = 1.0;
-                p1a[k] = R[k].t1;
-                p1b[k] = R[k].t2;
                 if (m > 0)
                 {
                     cell_seed(R[k], A.sg[2 * m], (int)A.sg[2 * m + 1], u1, u2,
@@ -923,10 +954,15 @@ __global__ void __launch_bounds__(CELL_WARPS * 32, K == 1 ? 3 : 2)
                 // zonal: un-normalised polynomials (sha_cell.c:880-960);
                 // the partial sums carry I_n0 / ct_n (k_sha_reduce applies
                 // ct_n)
+                ZonalRec Z[K];
+#pragma unroll
+                for (int k = 0; k < K; k++)
+                    Z[k].seed(R[k].t1, R[k].t2);
                 for (int j = 0; j < nchunks; j++)
                 {
                     const int cnt = (int)min((long long)LEG_CHUNK,
                                              ncol - (long long)j * LEG_CHUNK);
+                    stage_zonal(S, A, j, cnt, lane);
                     for (int half = 0; half < 2; half++)
                     {
                         const int ib = 32 * half;
@@ -943,36 +979,10 @@ __global__ void __launch_bounds__(CELL_WARPS * 32, K == 1 ? 3 : 2)
                                 (long long)j * LEG_CHUNK + ib + jj;
                             double vc = 0.0;
                             if (kk < ncol)
-                            {
-                                const double rct = 1.0 / A.tc[kk];
-                                const double4 z =
-                                    kk > 0 ? A.zn[kk]
-                                           : make_double4(0.0, 0.0, 0.0, 0.0);
 #pragma unroll
                                 for (int k = 0; k < K; k++)
-                                {
-                                    double in0;
-                                    if (kk == 0)
-                                        in0 = R[k].t2 - R[k].t1;
-                                    else
-                                    {
-                                        const double p2a =
-                                            z.x * (R[k].t1 * p1a[k]) -
-                                            z.y * p0a[k];
-                                        const double p2b =
-                                            z.x * (R[k].t2 * p1b[k]) -
-                                            z.y * p0b[k];
-                                        in0 = z.z * ((p2b - p0b[k]) -
-                                                     (p2a - p0a[k]));
-                                        p0a[k] = p1a[k];
-                                        p1a[k] = p2a;
-                                        p0b[k] = p1b[k];
-                                        p1b[k] = p2b;
-                                    }
-                                    vc = fma(in0 * rct,
+                                    vc = fma(Z[k].step(S, ib + jj, kk == 0),
                                              (kk & 1) ? amm[k] : amp[k], vc);
-                                }
-                            }
                             put(jj, vc, 0.0);
                         }
                         flush(i_l, prev);
@@ -1150,30 +1160,17 @@ __global__ void __launch_bounds__(CELL_WARPS * 32) k_shs_cell_sctr(CellArgs A)
             double rn = RR ? ratiom : 1.0;
             if (m == 0)
             {
-                double p0a = 1.0, p0b = 1.0, p1a = R.t1, p1b = R.t2;
+                ZonalRec Z;
+                Z.seed(R.t1, R.t2);
                 for (int j = 0; j < nchunks; j++)
                 {
                     const int cnt = (int)min((long long)LEG_CHUNK,
                                              ncol - (long long)j * LEG_CHUNK);
-                    stage_chunk(S, A, c0, m, j, cnt, lane);
+                    stage_zonal(S, A, j, cnt, lane);
                     for (int i = 0; i < cnt; i++)
                     {
-                        const long long n = (long long)j * LEG_CHUNK + i;
-                        double in0;
-                        if (n == 0)
-                            in0 = R.t2 - R.t1;
-                        else
-                        {
-                            const double4 z = A.zn[n];
-                            const double p2a = z.x * (R.t1 * p1a) - z.y * p0a;
-                            const double p2b = z.x * (R.t2 * p1b) - z.y * p0b;
-                            in0 = z.z * ((p2b - p0b) - (p2a - p0a));
-                            p0a = p1a;
-                            p1a = p2a;
-                            p0b = p1b;
-                            p1b = p2b;
-                        }
-                        const double v = (in0 / A.tc[c0 + n]) * rn;
+                        const double v =
+                            Z.step(S, i, j == 0 && i == 0) * rn;
                         if (RR)
                             rn *= rho;
                         a = fma(v, S.cs[i].x, a);
