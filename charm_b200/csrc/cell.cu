@@ -79,37 +79,56 @@ __device__ __forceinline__ Stage warp_stage_sha(unsigned char *base)
     return Stage{p, nullptr, p + LEG_CHUNK};
 }
 
-// Stages chunk j of order m: entries n = m + 64 j + i, i < cnt, of the
-// order's column (tb, cs) and (h_n beta_n, 1 / (n + 1)) in hn.  The warp
-// reads the stage only after the __syncwarp that ends this function.
-__device__ __forceinline__ void stage_chunk(const Stage &S, const CellArgs &A,
-                                            long long c0, long long m, int j,
-                                            int cnt, unsigned lane)
+// Chunk j of order m on its way into the stage: entries n = m + 64 j + i,
+// i < cnt, of the order's column (tb, cs) and of (h_n, 1 / (n + 1)), and the
+// factor that rescales the state between chunks.  A warp loads a chunk while
+// it works on the one before, so that the loads' latency is paid once per
+// item and not once per 64 degrees.
+struct ChunkRegs
 {
-    __syncwarp();
+    double2 b[2], c[2], h[2];
+    double mul;
+};
+
+template <bool CS>
+__device__ __forceinline__ void load_chunk(ChunkRegs &Q, const CellArgs &A,
+                                           long long c0, long long ncol,
+                                           long long m, int j, unsigned lane)
+{
     const long long off = (long long)j * LEG_CHUNK;
 #pragma unroll
     for (int h = 0; h < 2; h++)
     {
+        const long long i = off + (long long)lane + 32 * h;
+        Q.b[h] = Q.c[h] = Q.h[h] = make_double2(0.0, 0.0);
+        if (i < ncol)
+        {
+            Q.b[h] = A.tb[c0 + i];
+            Q.h[h] = A.hn[m + i];
+            if (CS)
+                Q.c[h] = A.cs[c0 + i];
+        }
+    }
+    Q.mul = j > 0 && off < ncol ? A.tmul[(size_t)m * A.ldmul + j] : 1.0;
+}
+
+// The loaded chunk into the stage: tb, cs and (h_n beta_n, 1 / (n + 1)) in
+// hn, zeros beyond the column.  The warp reads the stage only after the
+// __syncwarp that ends this function.
+template <bool CS>
+__device__ __forceinline__ void store_chunk(const Stage &S, const ChunkRegs &Q,
+                                            unsigned lane)
+{
+    __syncwarp();
+#pragma unroll
+    for (int h = 0; h < 2; h++)
+    {
         const int i = (int)lane + 32 * h;
-        if (i < cnt)
-        {
-            const double2 b = A.tb[c0 + off + i];
-            const double2 h = A.hn[m + off + i];
-            S.tb[i] = b;
-            if (S.cs)
-                S.cs[i] = A.cs[c0 + off + i];
-            // h_n beta_n formed once here instead of by every lane per
-            // degree
-            S.hn[i] = make_double2(h.x * b.x, h.y);
-        }
-        else
-        {
-            S.tb[i] = make_double2(0.0, 0.0);
-            if (S.cs)
-                S.cs[i] = make_double2(0.0, 0.0);
-            S.hn[i] = make_double2(0.0, 0.0);
-        }
+        S.tb[i] = Q.b[h];
+        if (CS)
+            S.cs[i] = Q.c[h];
+        // h_n beta_n formed once here instead of by every lane per degree
+        S.hn[i] = make_double2(Q.h[h].x * Q.b[h].x, Q.h[h].y);
     }
     __syncwarp();
 }
@@ -503,11 +522,15 @@ __global__ void __launch_bounds__(CELL_WARPS * 32) k_shs_cell(CellArgs A)
             cell_seed(R, sigma, g0, u1, u2, m,
                       valid ? A.imm[(size_t)m * np + p] : 0.0);
             bool any_scaled = __any_sync(0xffffffffu, (R.E1 | R.E2) != 0);
+            ChunkRegs Q;
+            load_chunk<true>(Q, A, c0, ncol, m, 0, lane);
             for (int j = 0; j < nchunks; j++)
             {
                 const int cnt = (int)min((long long)LEG_CHUNK,
                                          ncol - (long long)j * LEG_CHUNK);
-                stage_chunk(S, A, c0, m, j, cnt, lane);
+                store_chunk<true>(S, Q, lane);
+                const double mul = Q.mul;
+                load_chunk<true>(Q, A, c0, ncol, m, j + 1, lane);
                 int i0 = 0;
                 if (j == 0)
                 {
@@ -521,7 +544,7 @@ __global__ void __launch_bounds__(CELL_WARPS * 32) k_shs_cell(CellArgs A)
                     i0 = 1;
                 }
                 else
-                    R.scale(A.tmul[(size_t)m * A.ldmul + j]);
+                    R.scale(mul);
                 auto one = [&](int i, bool odd) {
                     const double beta = S.tb[i].x;
                     const double2 h = S.hn[i];
@@ -693,11 +716,15 @@ __global__ void __launch_bounds__(CELL_WARPS * 32) k_shs_cell2(CellArgs A)
             // the common boundary is renormalised through R[0]
             R[1].E2 = 0;
             bool any_scaled = __any_sync(0xffffffffu, sc);
+            ChunkRegs Q;
+            load_chunk<true>(Q, A, c0, ncol, m, 0, lane);
             for (int j = 0; j < nchunks; j++)
             {
                 const int cnt = (int)min((long long)LEG_CHUNK,
                                          ncol - (long long)j * LEG_CHUNK);
-                stage_chunk(S, A, c0, m, j, cnt, lane);
+                store_chunk<true>(S, Q, lane);
+                const double mul = Q.mul;
+                load_chunk<true>(Q, A, c0, ncol, m, j + 1, lane);
                 int i0 = 0;
                 if (j == 0)
                 {
@@ -716,7 +743,6 @@ __global__ void __launch_bounds__(CELL_WARPS * 32) k_shs_cell2(CellArgs A)
                 }
                 else
                 {
-                    const double mul = A.tmul[(size_t)m * A.ldmul + j];
                     R[0].scale(mul);
                     R[1].scale(mul);
                 }
@@ -991,11 +1017,15 @@ __global__ void __launch_bounds__(CELL_WARPS * 32, K == 1 ? 3 : 2)
                 stored = true;
                 continue;
             }
+            ChunkRegs Q;
+            load_chunk<false>(Q, A, c0, ncol, m, 0, lane);
             for (int j = 0; j < nchunks; j++)
             {
                 const int cnt = (int)min((long long)LEG_CHUNK,
                                          ncol - (long long)j * LEG_CHUNK);
-                stage_chunk(S, A, c0, m, j, cnt, lane);
+                store_chunk<false>(S, Q, lane);
+                const double mul = Q.mul;
+                load_chunk<false>(Q, A, c0, ncol, m, j + 1, lane);
                 if (j == 0)
                 {
                     // the seed step (see above)
@@ -1008,7 +1038,6 @@ __global__ void __launch_bounds__(CELL_WARPS * 32, K == 1 ? 3 : 2)
                 }
                 else
                 {
-                    const double mul = A.tmul[(size_t)m * A.ldmul + j];
 #pragma unroll
                     for (int k = 0; k < K; k++)
                         R[k].scale(mul);
@@ -1185,11 +1214,15 @@ __global__ void __launch_bounds__(CELL_WARPS * 32) k_shs_cell_sctr(CellArgs A)
                 R.J0 = 0.0;
                 R.J1 = scalbn(imm, g0);
                 bool any_scaled = __any_sync(0xffffffffu, (R.E1 | R.E2) != 0);
+                ChunkRegs Q;
+                load_chunk<true>(Q, A, c0, ncol, m, 0, lane);
                 for (int j = 0; j < nchunks; j++)
                 {
                     const int cnt = (int)min((long long)LEG_CHUNK,
                                              ncol - (long long)j * LEG_CHUNK);
-                    stage_chunk(S, A, c0, m, j, cnt, lane);
+                    store_chunk<true>(S, Q, lane);
+                    const double mul = Q.mul;
+                    load_chunk<true>(Q, A, c0, ncol, m, j + 1, lane);
                     int i = 0;
                     if (j == 0)
                     {
@@ -1201,7 +1234,7 @@ __global__ void __launch_bounds__(CELL_WARPS * 32) k_shs_cell_sctr(CellArgs A)
                         i = 1;
                     }
                     else
-                        R.scale(A.tmul[(size_t)m * A.ldmul + j]);
+                        R.scale(mul);
 #pragma unroll 4
                     for (; i < cnt; i++)
                     {

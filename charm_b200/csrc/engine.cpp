@@ -4059,8 +4059,10 @@ Status shs_cell_grid(Context &c, const charm_cell *cell, const CoefIn &in,
     A.nmax = (long long)nmax;
     A.npairs = np;
     // two adjacent pairs per lane when the rows are aligned (each pair of
-    // rows shares a boundary) and there are enough pairs
-    bool shared = np >= 512;
+    // rows shares a boundary) and there are enough pairs: one pair and two
+    // per lane took 55 and 76 us at 256 pairs, 117 and 134 at 360, 261 and
+    // 270 at 512, 689 and 614 at 720
+    bool shared = np >= 600;
     for (int p = 0; shared && p + 1 < np; p += 2)
         shared = cell->latmin[P.row_n[p]] == cell->latmax[P.row_n[p + 1]];
     A.ntiles = shared ? (np + 63) / 64 : (np + 31) / 32;
@@ -4331,11 +4333,14 @@ Status sha_cell_grid(Context &c, const charm_cell *cell, const double *f_host,
     const long long T = (long long)(nmax + 1) * (nmax + 2) / 2;
     // two cell-row pairs per lane once there are enough of them; adjacent
     // ones (pairs 2l, 2l + 1) when each such pair of rows shares a
-    // boundary, which the kernel then carries once
-    const int K = np >= 512 ? 2 : 1;
-    bool shared = K == 2;
+    // boundary, which the kernel then carries once.  One pair and two with
+    // the common boundary took 77 and 86 us at 256 pairs, 173 and 134 at
+    // 360, 430 and 320 at 512: the wider lanes also halve the traffic of the
+    // sums over the lanes, which bounds the kernel
+    bool shared = np >= 320;
     for (int p = 0; shared && p + 1 < np; p += 2)
         shared = cell->latmin[P.row_n[p]] == cell->latmax[P.row_n[p + 1]];
+    const int K = shared || np >= 512 ? 2 : 1;
     const int ntiles = (np + 32 * K - 1) / (32 * K);
     const long long slots = (long long)c.num_sms * 8 * 4;
     long long G = std::max<long long>(1, (2 * slots + nmax) / (nmax + 1));
