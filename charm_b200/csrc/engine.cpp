@@ -3290,7 +3290,8 @@ Status sctr_adjoint(Context &c, const charm_point *pnt, const double *g_host,
     Tabs tab;
     CB_TRY(tables(c, (long long)nmax, &tab));
     double *dpts = nullptr;
-    CB_TRY(dbuf(c, "sctr_pts", 3 * npt + (d_g ? 0 : npt), &dpts));
+    // latitudes, longitudes, radii, host weights; four constants per point
+    CB_TRY(dbuf(c, "sctr_pts", 8 * npt, &dpts));
     CB_CUDA(cudaMemcpyAsync(dpts, pnt->lat, npt * 8, cudaMemcpyHostToDevice,
                             c.stream), st);
     CB_CUDA(cudaMemcpyAsync(dpts + npt, pnt->lon, npt * 8,
@@ -3342,8 +3343,8 @@ Status sctr_adjoint(Context &c, const charm_point *pnt, const double *g_host,
                                         (long long)c.num_sms * 8);
     {
         Scope sc(c, TIMER_SCTR);
-        CB_CUDA(launch_sha_points(A, r_eq ? 1 : 2, K, std::max(grid, 1),
-                                  c.stream), st);
+        CB_CUDA(launch_sha_points(A, !r_eq, dpts + 4 * npt, K,
+                                  std::max(grid, 1), c.stream), st);
     }
     const long long Ts = (long long)(shc_nmax + 1) * (shc_nmax + 2) / 2;
     double *oc = d_c, *os = d_s;

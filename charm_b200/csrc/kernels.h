@@ -185,12 +185,15 @@ struct ShaGridArgs
     unsigned long long *counter;
     unsigned *status;
     // scattered points instead of grid pairs (adjoint of the scattered
-    // synthesis): npairs counts points, and these replace t, u, F, cw_*
+    // synthesis): npairs counts points, and these replace F, cw_*
     const double *lat;
     const double *lon;
     const double *r;       // radius per point (read when r != R)
     const double *g;       // weight of each point's value
     double R;              // reference radius of the coefficients
+    // filled by launch_sha_points (as t and u are)
+    const double *rho;     // R / r
+    const double *gs;      // g / rho^2
 };
 
 // Grid analysis with the two-degree recurrence (sha_two.cu); fields as
@@ -442,10 +445,10 @@ cudaError_t launch_lon_direct(int npar, int nlat, int nlon, long long nmax,
                               double *f, cudaStream_t st);
 cudaError_t launch_sha_grid(const ShaGridArgs &A, int K, int grid,
                             cudaStream_t st);
-// src: 0 grid pairs, 1 scattered points on the sphere r = R, 2 scattered
-// points with their own radii
-cudaError_t launch_sha_points(const ShaGridArgs &A, int src, int K, int grid,
-                              cudaStream_t st);
+// scattered points, with their own radii if rr; consts: 4 words per point of
+// scratch for what the kernel reads of every point (A points there after)
+cudaError_t launch_sha_points(ShaGridArgs &A, bool rr, double *consts, int K,
+                              int grid, cudaStream_t st);
 // k_sha_reduce for the orders [m_lo, m_hi) only
 cudaError_t launch_sha_reduce_orders(long long nmax, long long shc_nmax,
                                      int ngroups, long long T,
