@@ -40,6 +40,7 @@
 // MMAs of the chunk and commits them to an mbarrier, so the tensor cores
 // work on chunk j while the threads prepare chunk j + 1; epilogue warps
 // drain an item's accumulators while the next item is prepared.
+#include <algorithm>
 #include <cstdint>
 #include <type_traits>
 
@@ -321,7 +322,11 @@ __global__ void k_tc_colexp_grad(ShsTcPrep P)
 }
 
 // Digit tiles of every (order, chunk): [parity][digit][32 columns x 32 B].
-// One block per order, thread = (parity, column, 16-degree half).
+// Thread = (parity, column, 16-degree half).  Bound by the latency of the
+// coefficient loads, chunk after chunk: with one block per order the launch
+// waited for the longest orders, so an order's chunks are dealt to up to 8
+// blocks.  All preparation of 20 sets at nmax 1000 took 229 us with one block
+// per order, 149 with 2, 141 with 4, 133 with 8, 132 with 16.
 __global__ void __launch_bounds__(128) k_tc_bdigits(ShsTcPrep P)
 {
     const long long m = blockIdx.x;
@@ -346,7 +351,7 @@ __global__ void __launch_bounds__(128) k_tc_bdigits(ShsTcPrep P)
     const double sc = pow2i(54 - P.ecol[m * TC_COLS + col]);
     const long long nch = (P.nmax - m + TC_CH) / TC_CH;
     unsigned char *base = P.bdig + (size_t)P.chunk0[m] * TC_BSTAGE;
-    for (long long j = 0; j < nch; j++)
+    for (long long j = blockIdx.y; j < nch; j += gridDim.y)
     {
         unsigned w[TC_D][4];
 #pragma unroll
@@ -1223,7 +1228,9 @@ cudaError_t launch_tc_prep(const ShsTcPrep &P, cudaStream_t st)
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess)
         return e;
-    k_tc_bdigits<<<(unsigned)(P.nmax + 1), 128, 0, st>>>(P);
+    const unsigned nch = (unsigned)((P.nmax + TC_CH) / TC_CH);
+    k_tc_bdigits<<<dim3((unsigned)(P.nmax + 1), std::min(nch, 8u)), 128, 0,
+                   st>>>(P);
     return cudaGetLastError();
 }
 
