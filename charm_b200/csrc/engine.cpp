@@ -1277,7 +1277,7 @@ int choose_k_two(int n2, int mode)
 // Latitude pairs per lane of the analysis kernels.  Wider tiles amortise
 // the per-degree table load and the transpose-reduce over more latitudes but
 // lower the resident warps (sha_grid.cu, sha_two.cu); CHARM_B200_SHA_K (1, 2,
-// 4, 6 or 8) overrides the choice for tuning.
+// 4, 6 or 8; 1 to 8 for the two-degree kernel) overrides the choice for tuning.
 int choose_k_sha(long long npairs, bool two = false)
 {
     static const int forced = [] {

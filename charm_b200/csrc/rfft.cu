@@ -17,9 +17,10 @@
 //     a circular convolution of length M >= 2H - 1, M = 2^a 3^b, evaluated
 //     as FFT_M, a pointwise product with the precomputed FFT_M of the chirp,
 //     and a second FFT_M (conjugated in and out, which inverts it);
-//   * FFT_M by in-place Stockham autosort passes (radix 8, 4, 2 and 3 in
-//     the run-time plans; 16, 16, 18 for M = 4608 and 16, 16, 9, 4 for
-//     M = 9216 in the compile-time ones): every thread holds V values
+//   * FFT_M by in-place Stockham autosort passes (two to four of radix 3 to
+//     18 in the compile-time plans, CT_PLANS in rfft.cuh; radix 8, 4, 2 and
+//     3 in the run-time plans, which the kernel spectra, odd rows and the
+//     clusters without a fixed length use): every thread holds V values
 //     across the barrier that separates the loads of a pass from its
 //     stores, so one buffer of M values suffices.  The first pass reads its
 //     inputs straight from global memory (with the chirp applied; the zero

@@ -9,7 +9,9 @@
 // transpose-reduce leaves lane l with the warp total of degree n0 + l,
 // which is added to the group's partial column (plain read-modify-write:
 // the warp owns it).  k_sha_reduce (tables.cu) sums the groups in a fixed
-// order and applies ct_n, so results are deterministic.
+// order and applies ct_n, so results are deterministic.  Serves the grids
+// below the line at which sha_two.cu is faster (TWO_MIN_NMAX_SHA in
+// engine.cpp), and the allocation-free entry point.
 //
 // The same kernel computes the adjoint of the scattered-point synthesis
 // (src/shs/shs_point_sctr.c:86-728) with respect to the coefficients: the

@@ -12,6 +12,11 @@
 // for the potential.  The north/south symmetry
 // P_nm(-t) = (-1)^(n+m) P_nm(t) is used by keeping even and odd (n+m)
 // partial sums; the parity of every step is a compile-time constant.
+//
+// Serves what shs_two.cu does not take (two_pairs and TWO_MIN_NMAX in
+// engine.cpp): low degrees, grids whose rows have their own radii or whose
+// latitudes are not ordered by distance from the equator, and the rows at
+// the poles, whose horizontal derivatives are singular.
 #include <cstdint>
 #include <type_traits>
 
