@@ -139,7 +139,7 @@ __device__ __forceinline__ void store_chunk(const Stage &S, const ChunkRegs &Q,
 // the longest chain of a launch: with the table loads and the division by
 // ct_n in their loop over the degrees, they alone kept the kernels of nmax
 // 719 (361 pairs of rows) at 249 us of synthesis and 265 us of analysis; with
-// the stage these take 117 and 181.
+// the stage these take 117 and 181 (134 with two pairs of rows per lane).
 __device__ __forceinline__ void stage_zonal(const Stage &S, const CellArgs &A,
                                             int j, int cnt, unsigned lane)
 {
