@@ -413,14 +413,22 @@ struct RfftArgs
     int nbatch;
 };
 
-// the plans of rfft_ct*.cu; cudaErrorInvalidConfiguration: not in the file
-cudaError_t launch_rfft_ct0(const RfftArgs &A, bool inverse, cudaStream_t st);
-cudaError_t launch_rfft_ct1(const RfftArgs &A, bool inverse, cudaStream_t st);
-cudaError_t launch_rfft_ct2(const RfftArgs &A, bool inverse, cudaStream_t st);
-cudaError_t launch_rfft_ct3(const RfftArgs &A, bool inverse, cudaStream_t st);
-cudaError_t launch_rfft_ct4(const RfftArgs &A, bool inverse, cudaStream_t st);
-cudaError_t launch_rfft_ct5(const RfftArgs &A, bool inverse, cudaStream_t st);
-cudaError_t launch_rfft_ct6(const RfftArgs &A, bool inverse, cudaStream_t st);
+// the plans of rfft_ct*.cu: false when the length is not in the file, else the
+// launch's error in *e
+bool launch_rfft_ct0(const RfftArgs &A, bool inverse, cudaStream_t st,
+                     cudaError_t *e);
+bool launch_rfft_ct1(const RfftArgs &A, bool inverse, cudaStream_t st,
+                     cudaError_t *e);
+bool launch_rfft_ct2(const RfftArgs &A, bool inverse, cudaStream_t st,
+                     cudaError_t *e);
+bool launch_rfft_ct3(const RfftArgs &A, bool inverse, cudaStream_t st,
+                     cudaError_t *e);
+bool launch_rfft_ct4(const RfftArgs &A, bool inverse, cudaStream_t st,
+                     cudaError_t *e);
+bool launch_rfft_ct5(const RfftArgs &A, bool inverse, cudaStream_t st,
+                     cudaError_t *e);
+bool launch_rfft_ct6(const RfftArgs &A, bool inverse, cudaStream_t st,
+                     cudaError_t *e);
 
 // Size of the fixed device scratch of the allocation-free analysis
 // (sha_static.cu) and the largest degree it serves.

@@ -401,6 +401,21 @@ cudaError_t launch_rfftc_tables(RfftArgs &A, double2 *tw, double2 *twM,
 
 cudaError_t launch_rfft(const RfftArgs &A, bool inverse, cudaStream_t st)
 {
+    // the blocks of a batch are the grid's y dimension, 65535 at most
+    constexpr int MAX_BATCH = 65535;
+    if (A.batch && A.nbatch > MAX_BATCH)
+    {
+        for (int k = 0; k < A.nbatch; k += MAX_BATCH)
+        {
+            RfftArgs B = A;
+            B.batch = A.batch + k;
+            B.nbatch = A.nbatch - k < MAX_BATCH ? A.nbatch - k : MAX_BATCH;
+            const cudaError_t e = launch_rfft(B, inverse, st);
+            if (e != cudaSuccess)
+                return e;
+        }
+        return cudaSuccess;
+    }
     const unsigned grid = (unsigned)A.nrows;
     const unsigned ny = A.batch ? (unsigned)A.nbatch : 1u;
     if (grid == 0 || ny == 0)
@@ -458,17 +473,15 @@ cudaError_t launch_rfft(const RfftArgs &A, bool inverse, cudaStream_t st)
     // Bluestein: every length has its plan fixed at compile time
     if (!A.direct)
     {
-        static cudaError_t (*const group[])(const RfftArgs &, bool,
-                                            cudaStream_t) = {
+        static bool (*const group[])(const RfftArgs &, bool, cudaStream_t,
+                                     cudaError_t *) = {
             launch_rfft_ct0, launch_rfft_ct1, launch_rfft_ct2,
             launch_rfft_ct3, launch_rfft_ct4, launch_rfft_ct5,
             launch_rfft_ct6};
+        cudaError_t e = cudaSuccess;
         for (auto fn : group)
-        {
-            const cudaError_t e = fn(A, inverse, st);
-            if (e != cudaErrorInvalidConfiguration)
+            if (fn(A, inverse, st, &e))
                 return e;
-        }
     }
     // direct transforms, and the one length (6144) without an even last pass
     const dim3 g2(grid, ny);

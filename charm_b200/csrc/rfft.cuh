@@ -1034,8 +1034,7 @@ __global__ void RFFT_BOUNDS(RFFT_NR) k_rfft_inv(RfftArgs A)
 }
 
 
-// launch of the one-CTA kernels with the compile-time plan M, per group of
-// plans; cudaErrorInvalidConfiguration when M is not in the group
+// launch of the one-CTA kernels with the compile-time plan MC
 template <int MC>
 static cudaError_t rfft_ct_launch(const RfftArgs &A, bool inverse,
                                   cudaStream_t st)

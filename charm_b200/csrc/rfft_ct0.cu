@@ -4,16 +4,17 @@
 namespace cb
 {
 
-cudaError_t launch_rfft_ct0(const RfftArgs &A, bool inverse, cudaStream_t st)
+bool launch_rfft_ct0(const RfftArgs &A, bool inverse, cudaStream_t st,
+                     cudaError_t *e)
 {
     switch (A.M)
     {
-    case 64: return rfft_ct_launch<64>(A, inverse, st);
-    case 128: return rfft_ct_launch<128>(A, inverse, st);
-    case 192: return rfft_ct_launch<192>(A, inverse, st);
-    case 256: return rfft_ct_launch<256>(A, inverse, st);
-    case 384: return rfft_ct_launch<384>(A, inverse, st);
-    default: return cudaErrorInvalidConfiguration;
+    case 64: *e = rfft_ct_launch<64>(A, inverse, st); return true;
+    case 128: *e = rfft_ct_launch<128>(A, inverse, st); return true;
+    case 192: *e = rfft_ct_launch<192>(A, inverse, st); return true;
+    case 256: *e = rfft_ct_launch<256>(A, inverse, st); return true;
+    case 384: *e = rfft_ct_launch<384>(A, inverse, st); return true;
+    default: return false;
     }
 }
 

@@ -4,15 +4,16 @@
 namespace cb
 {
 
-cudaError_t launch_rfft_ct1(const RfftArgs &A, bool inverse, cudaStream_t st)
+bool launch_rfft_ct1(const RfftArgs &A, bool inverse, cudaStream_t st,
+                     cudaError_t *e)
 {
     switch (A.M)
     {
-    case 512: return rfft_ct_launch<512>(A, inverse, st);
-    case 576: return rfft_ct_launch<576>(A, inverse, st);
-    case 768: return rfft_ct_launch<768>(A, inverse, st);
-    case 1024: return rfft_ct_launch<1024>(A, inverse, st);
-    default: return cudaErrorInvalidConfiguration;
+    case 512: *e = rfft_ct_launch<512>(A, inverse, st); return true;
+    case 576: *e = rfft_ct_launch<576>(A, inverse, st); return true;
+    case 768: *e = rfft_ct_launch<768>(A, inverse, st); return true;
+    case 1024: *e = rfft_ct_launch<1024>(A, inverse, st); return true;
+    default: return false;
     }
 }
 

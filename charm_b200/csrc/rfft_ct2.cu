@@ -4,14 +4,15 @@
 namespace cb
 {
 
-cudaError_t launch_rfft_ct2(const RfftArgs &A, bool inverse, cudaStream_t st)
+bool launch_rfft_ct2(const RfftArgs &A, bool inverse, cudaStream_t st,
+                     cudaError_t *e)
 {
     switch (A.M)
     {
-    case 1152: return rfft_ct_launch<1152>(A, inverse, st);
-    case 1536: return rfft_ct_launch<1536>(A, inverse, st);
-    case 1728: return rfft_ct_launch<1728>(A, inverse, st);
-    default: return cudaErrorInvalidConfiguration;
+    case 1152: *e = rfft_ct_launch<1152>(A, inverse, st); return true;
+    case 1536: *e = rfft_ct_launch<1536>(A, inverse, st); return true;
+    case 1728: *e = rfft_ct_launch<1728>(A, inverse, st); return true;
+    default: return false;
     }
 }
 

@@ -4,14 +4,15 @@
 namespace cb
 {
 
-cudaError_t launch_rfft_ct3(const RfftArgs &A, bool inverse, cudaStream_t st)
+bool launch_rfft_ct3(const RfftArgs &A, bool inverse, cudaStream_t st,
+                     cudaError_t *e)
 {
     switch (A.M)
     {
-    case 2048: return rfft_ct_launch<2048>(A, inverse, st);
-    case 2304: return rfft_ct_launch<2304>(A, inverse, st);
-    case 3072: return rfft_ct_launch<3072>(A, inverse, st);
-    default: return cudaErrorInvalidConfiguration;
+    case 2048: *e = rfft_ct_launch<2048>(A, inverse, st); return true;
+    case 2304: *e = rfft_ct_launch<2304>(A, inverse, st); return true;
+    case 3072: *e = rfft_ct_launch<3072>(A, inverse, st); return true;
+    default: return false;
     }
 }
 

@@ -4,14 +4,15 @@
 namespace cb
 {
 
-cudaError_t launch_rfft_ct4(const RfftArgs &A, bool inverse, cudaStream_t st)
+bool launch_rfft_ct4(const RfftArgs &A, bool inverse, cudaStream_t st,
+                     cudaError_t *e)
 {
     switch (A.M)
     {
-    case 3456: return rfft_ct_launch<3456>(A, inverse, st);
-    case 4096: return rfft_ct_launch<4096>(A, inverse, st);
-    case 4608: return rfft_ct_launch<4608>(A, inverse, st);
-    default: return cudaErrorInvalidConfiguration;
+    case 3456: *e = rfft_ct_launch<3456>(A, inverse, st); return true;
+    case 4096: *e = rfft_ct_launch<4096>(A, inverse, st); return true;
+    case 4608: *e = rfft_ct_launch<4608>(A, inverse, st); return true;
+    default: return false;
     }
 }
 

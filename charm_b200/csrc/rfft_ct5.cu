@@ -4,13 +4,14 @@
 namespace cb
 {
 
-cudaError_t launch_rfft_ct5(const RfftArgs &A, bool inverse, cudaStream_t st)
+bool launch_rfft_ct5(const RfftArgs &A, bool inverse, cudaStream_t st,
+                     cudaError_t *e)
 {
     switch (A.M)
     {
-    case 5184: return rfft_ct_launch<5184>(A, inverse, st);
-    case 6912: return rfft_ct_launch<6912>(A, inverse, st);
-    default: return cudaErrorInvalidConfiguration;
+    case 5184: *e = rfft_ct_launch<5184>(A, inverse, st); return true;
+    case 6912: *e = rfft_ct_launch<6912>(A, inverse, st); return true;
+    default: return false;
     }
 }
 

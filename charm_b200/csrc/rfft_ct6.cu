@@ -4,13 +4,14 @@
 namespace cb
 {
 
-cudaError_t launch_rfft_ct6(const RfftArgs &A, bool inverse, cudaStream_t st)
+bool launch_rfft_ct6(const RfftArgs &A, bool inverse, cudaStream_t st,
+                     cudaError_t *e)
 {
     switch (A.M)
     {
-    case 8192: return rfft_ct_launch<8192>(A, inverse, st);
-    case 9216: return rfft_ct_launch<9216>(A, inverse, st);
-    default: return cudaErrorInvalidConfiguration;
+    case 8192: *e = rfft_ct_launch<8192>(A, inverse, st); return true;
+    case 9216: *e = rfft_ct_launch<9216>(A, inverse, st); return true;
+    default: return false;
     }
 }
 
