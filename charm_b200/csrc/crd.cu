@@ -18,7 +18,7 @@ __device__ __forceinline__ bool nearly_zero(double a, double eps)
 }
 
 __global__ void k_gl_nodes(unsigned long nmax, double *lat, double *w,
-                           unsigned *status)
+                           unsigned *status, unsigned long maxit)
 {
     const unsigned long L = nmax + 1;
     const size_t nlat = L;
@@ -46,8 +46,8 @@ __global__ void k_gl_nodes(unsigned long nmax, double *lat, double *w,
         z1 = z;
         z -= p1 / pp;
         it++;
-    } while (fabs(z - z1) > DBL_EPSILON && it < 1000);
-    if (it >= 1000 || !isfinite(z))
+    } while (fabs(z - z1) > DBL_EPSILON && it < maxit);
+    if (it >= maxit || !isfinite(z))
         atomicOr(status, DEV_ERR_BAD_ARGS);
     size_t north = i, south = nlat - 1 - i;
     lat[south] = -asin(z);
@@ -101,11 +101,12 @@ __global__ void k_dh_nodes(unsigned long nmax, double *lat, double *w)
 }
 
 cudaError_t launch_gl_nodes(unsigned long nmax, double *lat, double *w,
-                            unsigned *status, cudaStream_t st)
+                            unsigned *status, unsigned long maxit,
+                            cudaStream_t st)
 {
     size_t nnorth = (nmax + 2) / 2;
     k_gl_nodes<<<(int)((nnorth + 127) / 128), 128, 0, st>>>(nmax, lat, w,
-                                                             status);
+                                                             status, maxit);
     return cudaGetLastError();
 }
 

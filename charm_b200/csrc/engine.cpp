@@ -99,8 +99,8 @@ struct Context
     // orders, EV_START the start of the copy stream after the work already
     // on the compute stream
     cudaEvent_t band_ev[16] = {};
-    // page-locked status word: the grid calls' kernels write it directly, the
-    // others' device word is copied here at the end of a call
+    // page-locked status words: the grid calls' kernels write [0] directly, the
+    // others' device word is copied to [1] at the end of a call
     unsigned *h_status = nullptr;
     // a sequence of grid calls whose synchronisations wait for its end
     // (gfm_global_impl): each call stages its uploads in a page-locked slot
@@ -1391,18 +1391,21 @@ Status finish(Context &c, unsigned *d_status)
     Status st;
     if (c.capturing)
         return st;   // read by batch_graph_launch after each replay
-    if (c.deferred)
+    if (c.deferred && d_status == c.h_status)
         return st;   // at the end of the sequence
+    unsigned *word = c.h_status;
     if (d_status != c.h_status)
     {
         // into page-locked memory, so the copy is queued like a kernel and
-        // the one synchronisation below covers both
-        *c.h_status = 0u;
-        CB_CUDA(cudaMemcpyAsync(c.h_status, d_status, sizeof(unsigned),
+        // the one synchronisation below covers both; not into the word that
+        // collects the status of a deferred sequence
+        word = c.h_status + 1;
+        *word = 0u;
+        CB_CUDA(cudaMemcpyAsync(word, d_status, sizeof(unsigned),
                                 cudaMemcpyDeviceToHost, c.stream), st);
     }
     CB_CUDA(cudaStreamSynchronize(c.stream), st);
-    const unsigned h_status = *static_cast<volatile unsigned *>(c.h_status);
+    const unsigned h_status = *static_cast<volatile unsigned *>(word);
     if (c.timing)
         resolve_timers(c);
     if (h_status)
@@ -4829,12 +4832,7 @@ Status gfm_global_impl(Context &c, const GfmArgs &g)
                                   g.pmax, i, imax));
         }
     }
-    if (g.pot)
-    {
-        CB_TRY(download_tri(c, dpot, np, g.pot->c));
-        CB_TRY(download_tri(c, dpot + Tp, np, g.pot->s));
-        CB_CUDA(cudaStreamSynchronize(c.stream), st);
-    }
+    // (before the caller's potential is written)
     if (defer.on)
     {
         c.deferred = false;
@@ -4843,6 +4841,9 @@ Status gfm_global_impl(Context &c, const GfmArgs &g)
     }
     if (g.pot)
     {
+        CB_TRY(download_tri(c, dpot, np, g.pot->c));
+        CB_TRY(download_tri(c, dpot + Tp, np, g.pot->s));
+        CB_CUDA(cudaStreamSynchronize(c.stream), st);
         g.pot->mu = gm;
         g.pot->r = g.R;
     }
@@ -5745,8 +5746,15 @@ Status quad_nodes(int type, unsigned long nmax, double *lat, double *w)
     CB_TRY(status_words(c, &d_status, &d_counter));
     {
         Scope sc(c, TIMER_PREP);
+        // CHarm's limit of the Newton iterations (CHARM_B200_GL_MAXIT lowers
+        // it, to see how a failure is reported)
+        unsigned long maxit = 1000;
+        if (const char *e = std::getenv("CHARM_B200_GL_MAXIT"))
+            if (const unsigned long v = std::strtoul(e, nullptr, 10))
+                maxit = std::min(maxit, v);
         if (type == CHARM_CRD_POINT_GRID_GL)
-            CB_CUDA(launch_gl_nodes(nmax, d, d + nlat, d_status, c.stream), st);
+            CB_CUDA(launch_gl_nodes(nmax, d, d + nlat, d_status, maxit,
+                                    c.stream), st);
         else
             CB_CUDA(launch_dh_nodes(nmax, d, d + nlat, c.stream), st);
     }

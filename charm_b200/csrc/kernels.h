@@ -491,7 +491,8 @@ cudaError_t launch_sha_two(const ShaTwoArgs &A, int K, int grid,
 cudaError_t launch_two_reduce(const TwoReduceArgs &A, long long m_lo,
                               long long m_hi, cudaStream_t st);
 cudaError_t launch_gl_nodes(unsigned long nmax, double *lat, double *w,
-                            unsigned *status, cudaStream_t st);
+                            unsigned *status, unsigned long maxit,
+                            cudaStream_t st);
 cudaError_t launch_dh_nodes(unsigned long nmax, double *lat, double *w,
                             cudaStream_t st);
 cudaError_t launch_fp64_probe(long long iters, int blocks, int threads,
