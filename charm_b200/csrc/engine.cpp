@@ -122,6 +122,9 @@ struct Context
     long long tab_nmax[TAB_SLOTS] = {-1, -1, -1};
     unsigned long long tab_used[TAB_SLOTS] = {};
     bool tab_two[TAB_SLOTS] = {};   // the slot's two-degree tables are built
+    // the call at hand uses the two-degree recurrence; must not (its buffers
+    // do not fit); was run again without it (or_one_degree)
+    bool two_live = false, one_degree = false, fell_back = false;
     unsigned long long tab_clock = 0;
     // bumped whenever a cached device buffer is (re)allocated or a cached
     // table is rewritten: a captured graph reads these by address, so it
@@ -252,6 +255,7 @@ Status init(Context &c)
 {
     Status st;
     int dev = 0;
+    c.two_live = false;
     CB_CUDA(cudaGetDevice(&dev), st);
     if (c.ready)
     {
@@ -298,6 +302,54 @@ Status init(Context &c)
     return st;
 }
 
+// Frees what the two-degree recurrence keeps on the device (tables, its forms
+// of the coefficients, power tables, the equatorial sums): no call needs it
+// to be served.  True when there was any.
+bool two_release(Context &c)
+{
+    static const char *const names[] = {"tab_ab", "tab_ag",   "tab_kw",
+                                        "tab_sm", "two_cs",   "two_batch_cs",
+                                        "geo_pow", "sha_part1"};
+    bool any = false;
+    for (auto &kv : c.bufs)
+        for (const char *n : names)
+            if (kv.second.p && kv.first.rfind(n, 0) == 0)
+            {
+                if (!any)
+                    cudaStreamSynchronize(c.stream);
+                any = true;
+                cudaFree(kv.second.p);
+                kv.second = DevBuf{};
+                break;
+            }
+    for (bool &b : c.tab_two)
+        b = false;
+    if (any)
+        c.epoch++;
+    return any;
+}
+
+// Runs a grid call; where the device memory does not hold what the two-degree
+// recurrence needs beside the rest, once more with the one-degree kernels
+// alone, whose buffers are a half to a tenth of its.
+template <typename F> Status or_one_degree(Context &c, const F &call)
+{
+    Status st = call();
+    const bool two = c.two_live;
+    c.two_live = false;
+    if (st.code != CHARM_EMEM || !two || c.one_degree || c.capturing)
+        return st;
+    struct Off
+    {
+        Context &c;
+        ~Off() { c.one_degree = false; }
+    } off{c};
+    cudaStreamSynchronize(c.copy_stream);
+    two_release(c);
+    c.one_degree = c.fell_back = true;
+    return call();
+}
+
 Status buf(Context &c, const std::string &name, size_t bytes, void **out)
 {
     Status st;
@@ -320,9 +372,13 @@ Status buf(Context &c, const std::string &name, size_t bytes, void **out)
         size_t want = std::max<size_t>(bytes, 256);
         c.epoch++;
         cudaError_t e = cudaMalloc(&b.p, want);
+        // (the buffers that earlier calls left, where this one reads none)
+        if (e == cudaErrorMemoryAllocation && !c.two_live && two_release(c))
+            e = cudaMalloc(&b.p, want);
         if (e != cudaSuccess)
         {
             cudaGetLastError();
+            b.p = nullptr;
             st.code = CHARM_EMEM;
             st.msg = std::string(CHARM_ERR_MALLOC_FAILURE) +
                      " (device buffer \"" + name + "\", " +
@@ -1641,8 +1697,10 @@ Status grid_geometry(Context &c, const charm_point *pnt, const Pairs &P,
             G->r = r0;
         }
     }
-    if (!G->rr && nmax >= two_min && (!weights || np >= TWO_MIN_PAIRS_SHA))
+    if (!G->rr && nmax >= two_min && !c.one_degree &&
+        (!weights || np >= TWO_MIN_PAIRS_SHA))
         G->n2 = two_pairs(hlat, np, &G->polar);
+    c.two_live = G->n2 > 0;
     // nothing for k_geometry to do but the sines: they come from the host
     // (and for the pairs at a pole in any case, so that their noise is the
     // same with and without it)
@@ -1784,9 +1842,9 @@ int grid_bands(const Pairs &P, int nlat, int units, int per, int nb,
     return nb;
 }
 
-Status shs_grid(Context &c, const charm_point *pnt, const CoefIn &in,
-                unsigned long nmax, int kgrad, int dr, int dlat, int dlon,
-                double **f, double *d_f)
+Status shs_grid_run(Context &c, const charm_point *pnt, const CoefIn &in,
+                    unsigned long nmax, int kgrad, int dr, int dlat, int dlon,
+                    double **f, double *d_f)
 {
     Status st;
     const double thr = charm_glob_threshold, thr2 = charm_glob_threshold2;
@@ -1871,11 +1929,12 @@ Status shs_grid(Context &c, const charm_point *pnt, const CoefIn &in,
         !in.dc && !d_f &&
         shs_k_settled(c, kgrad, dr, dlat, variant, (long long)nmax, np);
     if (old_too)
-        CB_TRY(dbuf(c, "cs", (size_t)((nmax + 1) * (nmax + 2) / 2) *
-                                 (n2 > 0 ? fam.nfam : 1), &dcs));
+        CB_TRY(dbuf(c, n2 > 0 ? "two_cs1" : "cs",
+                    (size_t)((nmax + 1) * (nmax + 2) / 2) *
+                        (n2 > 0 ? fam.nfam : 1), &dcs));
     if (n2 > 0)
-        CB_TRY(dbuf(c, "cs2", (size_t)(2 * two_steps((long long)nmax)) *
-                                  fam.nfam, &dcs2));
+        CB_TRY(dbuf(c, "two_cs", (size_t)(2 * two_steps((long long)nmax)) *
+                                     fam.nfam, &dcs2));
     if (!in.dc)
     {
         CB_TRY(dbuf(c, "shc_in", (size_t)(2 * Ts), &raw));
@@ -2220,6 +2279,15 @@ Status shs_grid(Context &c, const charm_point *pnt, const CoefIn &in,
     return finish(c, d_status);
 }
 
+Status shs_grid(Context &c, const charm_point *pnt, const CoefIn &in,
+                unsigned long nmax, int kgrad, int dr, int dlat, int dlon,
+                double **f, double *d_f)
+{
+    return or_one_degree(c, [&] {
+        return shs_grid_run(c, pnt, in, nmax, kgrad, dr, dlat, dlon, f, d_f);
+    });
+}
+
 // ---------------------------------------------------------------------------
 // Scattered synthesis
 // ---------------------------------------------------------------------------
@@ -2468,10 +2536,11 @@ Status synth_rows(Context &c, const RfftArgs *rf, const RfftArgs *rfq,
 // item (set, order, latitude tile) stops at its set's own nmax.  kgrad 0:
 // potential, 1: grad1, 2: grad2, 3: all ten quantities (potential, grad1
 // x y z, grad2 xx xy xz yy yz zz, in CHarm's output order) per set.
-Status shs_batch(Context &c, const charm_point *pnt, size_t nsets,
-                 const unsigned long *nmax_v, const unsigned long *shc_nmax_v,
-                 const double *mu_v, double R, const double *const *d_c,
-                 const double *const *d_s, int kgrad, double *const *d_f)
+Status shs_batch_run(Context &c, const charm_point *pnt, size_t nsets,
+                     const unsigned long *nmax_v,
+                     const unsigned long *shc_nmax_v, const double *mu_v,
+                     double R, const double *const *d_c,
+                     const double *const *d_s, int kgrad, double *const *d_f)
 {
     Status st;
     const size_t nlat = pnt->nlat, nlon = pnt->nlon;
@@ -2499,12 +2568,9 @@ Status shs_batch(Context &c, const charm_point *pnt, size_t nsets,
                         (two ? fam.nfam : 1);
     const long long T2 = 2 * two_steps((long long)N) * fam.nfam;
     double2 *cs_all = nullptr, *cs2_all = nullptr;
-    if (old_too)
-        CB_TRY(dbuf(c, "batch_cs", (size_t)nsets * T, &cs_all));
-    if (n2 > 0)
-        CB_TRY(dbuf(c, "batch_cs2", (size_t)nsets * T2, &cs2_all));
-    for (size_t j = 0; j < nsets; j++)
-    {
+    // the kernels' forms of set j's coefficients, at place k of the buffers
+    auto scale = [&](size_t j, size_t k) -> Status {
+        Status s2;
         ScaleArgs S = fam;
         S.ntab = (long long)N;
         S.nmax = (long long)nmax_v[j];
@@ -2514,16 +2580,26 @@ Status shs_batch(Context &c, const charm_point *pnt, size_t nsets,
         S.tc = tab.tc;
         S.kw = tab.kw;
         S.rhop = G.rhop;
-        S.cs = cs_all ? cs_all + (size_t)j * T : nullptr;
-        S.cs2 = cs2_all ? cs2_all + (size_t)j * T2 : nullptr;
+        S.cs = cs_all ? cs_all + k * T : nullptr;
+        S.cs2 = cs2_all ? cs2_all + k * T2 : nullptr;
         const bool with = G.pending;
         Scope sc(c, TIMER_PREP);
         CB_CUDA(launch_two_scale(S, 0, S.nmax + 1, with ? &G.args : nullptr,
-                                 c.stream), st);
+                                 c.stream), s2);
         if (with)
             G.pending = false;
+        return s2;
+    };
+    // one-degree recurrence: every set now, for up to three passes over them;
+    // two-degree: per sub-batch below (up to 160 bytes per coefficient
+    // instead of 16, of all sets as much as half their output)
+    if (!two)
+    {
+        CB_TRY(dbuf(c, "batch_cs", nsets * (size_t)T, &cs_all));
+        for (size_t j = 0; j < nsets; j++)
+            CB_TRY(scale(j, j));
+        CB_TRY(geometry_launch(c, &G));
     }
-    CB_TRY(geometry_launch(c, &G));
     const RfftArgs *rf = nullptr, *rfq = nullptr;
     CB_TRY(row_fft(c, (long long)nlon, &rf));
     CB_TRY(row_fft_quarter(c, (long long)nlon, rf, &rfq));
@@ -2564,10 +2640,18 @@ Status shs_batch(Context &c, const charm_point *pnt, size_t nsets,
     {
         const int kg = kd.kgrad, npar = kd.npar;
         const int dd = kg;   // grad kinds: dr = dlat = dlon = kgrad
-        // sets per launch, bounded by the lumped-coefficient buffer (8 GB)
+        // sets per launch, bounded by the lumped-coefficient buffer and the
+        // two-degree forms of the coefficients (8 GB)
         const size_t per_set = (size_t)npar * nlat * ldf * sizeof(double2);
-        size_t bsz = std::max<size_t>(1, ((size_t)8 << 30) / per_set);
+        const size_t per_cs =
+            two ? (size_t)(T2 + (old_too ? T : 0)) * sizeof(double2) : 0;
+        size_t bsz = std::max<size_t>(1, ((size_t)8 << 30) /
+                                             (per_set + per_cs));
         bsz = std::min(bsz, nsets);
+        if (two)
+            CB_TRY(dbuf(c, "two_batch_cs", bsz * (size_t)T2, &cs2_all));
+        if (two && old_too)
+            CB_TRY(dbuf(c, "two_batch_cs1", bsz * (size_t)T, &cs_all));
         double2 *lc = nullptr;
         CB_TRY(dbuf(c, "batch_lumped", bsz * per_set / sizeof(double2), &lc));
         BatchSet *dsets = nullptr;
@@ -2581,9 +2665,12 @@ Status shs_batch(Context &c, const charm_point *pnt, size_t nsets,
         {
             const size_t nb = std::min(bsz, nsets - j0);
             long long items = 0;
+            for (size_t b = 0; two && b < nb; b++)
+                CB_TRY(scale(j0 + b, b));
             for (size_t b = 0; b < nb; b++)
             {
                 const size_t j = j0 + b;
+                const size_t k = two ? b : j;
                 double mur;
                 int dorder, npar_j;
                 mur_dorder(mu_v[j], G.r, ten ? 0 : kg, ten ? 0 : dd,
@@ -2598,8 +2685,8 @@ Status shs_batch(Context &c, const charm_point *pnt, size_t nsets,
                 }
                 hsets[b].nmax = (long long)nmax_v[j];
                 hsets[b].item0 = items;
-                hsets[b].cs1 = cs_all ? cs_all + j * T : nullptr;
-                hsets[b].cs = two ? cs2_all + j * T2 : hsets[b].cs1;
+                hsets[b].cs1 = cs_all ? cs_all + k * T : nullptr;
+                hsets[b].cs = two ? cs2_all + k * T2 : hsets[b].cs1;
                 hsets[b].out = lc + b * (per_set / sizeof(double2));
                 hsets[b].mur = mur;
                 hsets[b].polar_thr = polar_threshold(nmax_v[j]);
@@ -2756,6 +2843,17 @@ Status shs_batch(Context &c, const charm_point *pnt, size_t nsets,
     }
     (void)ncomp;
     return finish(c, d_status);
+}
+
+Status shs_batch(Context &c, const charm_point *pnt, size_t nsets,
+                 const unsigned long *nmax_v, const unsigned long *shc_nmax_v,
+                 const double *mu_v, double R, const double *const *d_c,
+                 const double *const *d_s, int kgrad, double *const *d_f)
+{
+    return or_one_degree(c, [&] {
+        return shs_batch_run(c, pnt, nsets, nmax_v, shc_nmax_v, mu_v, R, d_c,
+                             d_s, kgrad, d_f);
+    });
 }
 
 // ---------------------------------------------------------------------------
@@ -3378,10 +3476,11 @@ Status sctr_adjoint(Context &c, const charm_point *pnt, const double *g_host,
 // pair0 / pair1: with pair1 >= 0, only the latitude pairs [pair0, pair1)
 // of the grid's pairing (grid_pairs) enter the sums (a band of one
 // latitude-band-sharded analysis; device grids only).
-Status sha_grid(Context &c, const charm_point *pnt, const double *f_host,
-                const double *d_fin, unsigned long nmax, double mu, double R,
-                unsigned long shc_nmax, double *const *hc, double *const *hs,
-                double *d_c, double *d_s, int pair0 = 0, int pair1 = -1)
+Status sha_grid_run(Context &c, const charm_point *pnt, const double *f_host,
+                    const double *d_fin, unsigned long nmax, double mu,
+                    double R, unsigned long shc_nmax, double *const *hc,
+                    double *const *hs, double *d_c, double *d_s, int pair0,
+                    int pair1)
 {
     Status st;
     const size_t nlat = pnt->nlat, nlon = pnt->nlon;
@@ -3783,6 +3882,17 @@ Status sha_grid(Context &c, const charm_point *pnt, const double *f_host,
     }
     // res must stay alive until the copy ran: finish() synchronises
     return finish(c, d_status);
+}
+
+Status sha_grid(Context &c, const charm_point *pnt, const double *f_host,
+                const double *d_fin, unsigned long nmax, double mu, double R,
+                unsigned long shc_nmax, double *const *hc, double *const *hs,
+                double *d_c, double *d_s, int pair0 = 0, int pair1 = -1)
+{
+    return or_one_degree(c, [&] {
+        return sha_grid_run(c, pnt, f_host, d_fin, nmax, mu, R, shc_nmax, hc,
+                            hs, d_c, d_s, pair0, pair1);
+    });
 }
 
 // ---------------------------------------------------------------------------
@@ -5488,8 +5598,11 @@ Status batch_graph_create(const charm_point *pnt, size_t nsets,
                                  d_s, kgrad, d_f);
     };
     // a plain call first: checks the arguments, builds every table, plan,
-    // buffer and tuned choice the captured call then finds in place
+    // buffer and tuned choice the captured call then finds in place, and
+    // settles whether the two-degree recurrence fits the memory
+    c.fell_back = false;
     CB_TRY(run());
+    c.one_degree = c.fell_back;
     const bool timing = c.timing;
     c.timing = false;
     c.capturing = true;
@@ -5503,7 +5616,7 @@ Status batch_graph_create(const charm_point *pnt, size_t nsets,
         s2 = run();
         e = cudaStreamEndCapture(c.stream, &g);
     }
-    c.capturing = false;
+    c.capturing = c.one_degree = false;
     c.timing = timing;
     std::vector<void *> pins;
     pins.swap(c.capture_pins);
