@@ -32,6 +32,7 @@
 #include <vector>
 
 #include "kernels.h"
+#include "lat_pairs.h"
 
 namespace cb
 {
@@ -1612,38 +1613,7 @@ constexpr unsigned long TWO_MIN_NMAX_ONE = 400;
 // for the latitudes; DH1 520 58 against 68).
 constexpr unsigned long TWO_MIN_NMAX_SHA = 512;
 constexpr int TWO_MIN_PAIRS_SHA = 384;
-constexpr double TWO_NEAR = 0.05;      // |sin(lat)| (two.cuh)
 constexpr double POLE_COS = 1e-6;
-
-// Pairs that the two-degree recurrence may take: |lat| must not grow along
-// the pairs (so that neighbouring lanes are neighbouring latitudes and the
-// polar form of a 32-pair group fits all of it), from the first pair to the
-// first one within TWO_NEAR of the equator.  *polar: the leading pairs, in
-// whole groups of 32, poleward of 30 degrees.
-int two_pairs(const double *lat, int np, int *polar)
-{
-    const double near = std::asin(TWO_NEAR);
-    int n2 = np;
-    for (int p = 0; p < np; p++)
-    {
-        const double a = std::fabs(lat[p]);
-        if (p > 0 && !(a <= std::fabs(lat[p - 1])))
-            return 0;
-        if (!(a >= near) && n2 == np)
-            n2 = p;
-    }
-    // whole warps: the last up to 31 of them join the others when that leaves
-    // the others outside 0.8 TWO_NEAR
-    const int whole = (np - n2) / 32 * 32;
-    if (n2 < np && whole > 0 &&
-        std::fabs(lat[np - whole - 1]) >= std::asin(0.8 * TWO_NEAR))
-        n2 = np - whole;
-    int g = 0;
-    while (32 * (g + 1) <= n2 && std::fabs(lat[32 * g + 31]) >= PI / 6.0)
-        g++;
-    *polar = 32 * g;
-    return n2;
-}
 
 // weights (analysis): the rows' quadrature weights times cw are uploaded too.
 // r_eq: every row at the coefficients' radius R (nothing to fold); two_min:
