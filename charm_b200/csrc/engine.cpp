@@ -1667,18 +1667,20 @@ Status grid_geometry(Context &c, const charm_point *pnt, const Pairs &P,
             G->r = r0;
         }
     }
-    if (!G->rr && nmax >= two_min && !c.one_degree &&
+    const bool range = latitudes_in_range(hlat, np);
+    if (!G->rr && range && nmax >= two_min && !c.one_degree &&
         (!weights || np >= TWO_MIN_PAIRS_SHA))
         G->n2 = two_pairs(hlat, np, &G->polar);
     c.two_live = G->n2 > 0;
     // nothing for k_geometry to do but the sines: they come from the host
     // (and for the pairs at a pole in any case, so that their noise is the
-    // same with and without it)
+    // same with and without it, and for angles that are no latitudes)
     const bool plain = G->n2 == 0 && G->rho == 1.0;
     double *const ht = hlat + 4 * np, *const hu = hlat + 5 * np;
     while (G->npole < np && std::fabs(hlat[G->npole]) >= PI / 2 - POLE_COS)
         G->npole++;
-    for (int p = 0; p < (plain ? np : G->npole); p++)
+    const int given = range ? G->npole : np;
+    for (int p = 0; p < (plain ? np : given); p++)
         sincos(hlat[p], &ht[p], &hu[p]);
     void *dgeo = nullptr;
     CB_TRY(buf(c, "geo", up + (size_t)np * 3 * 8, &dgeo));
@@ -1710,7 +1712,7 @@ Status grid_geometry(Context &c, const charm_point *pnt, const Pairs &P,
     A.plain = plain ? 1 : 0;
     A.npairs = np;
     A.polar = G->polar;
-    A.given = G->npole;
+    A.given = given;
     A.lat = hlat;
     A.t = dt;
     A.u = dt + np;

@@ -8,6 +8,17 @@ namespace cb
 {
 
 constexpr double TWO_NEAR = 0.05;      // |sin(lat)| (two.cuh)
+// Latitudes of a sphere, with room for the rounding of one in degrees.  A
+// grid may hold any angles: beyond this the series of k_geometry do not serve.
+constexpr double LAT_MAX = 1.57079632679489661923 + 1e-6;
+
+inline bool latitudes_in_range(const double *lat, int np)
+{
+    for (int p = 0; p < np; p++)
+        if (!(std::fabs(lat[p]) <= LAT_MAX))
+            return false;
+    return true;
+}
 
 // Pairs that the two-degree recurrence may take: |lat| must not grow along
 // the pairs (so that neighbouring lanes are neighbouring latitudes and the
