@@ -1568,9 +1568,9 @@ Status coef_to_device(Context &c, const CoefIn &in, unsigned long nmax,
 struct GridGeo
 {
     int np = 0, n2 = 0, polar = 0;
-    // leading pairs at a pole (POLE_COS): the quantities with 1 / cos(lat)
-    // are rounding noise there, the same noise from every call only if one
-    // kernel forms it, the one-degree one
+    // leading pairs at a pole (POLE_COS): derivatives along the meridian, with
+    // their 1 / cos(lat), are rounding noise there, the same noise from every
+    // call only if one kernel forms it, the one-degree one
     int npole = 0;
     // one radius r for all rows, other than R: (R / r)^n is folded into the
     // coefficients (rhop), the call's factor is GM / r^(dorder + 1), and rr
@@ -1886,9 +1886,9 @@ Status shs_grid_run(Context &c, const charm_point *pnt, const CoefIn &in,
     Tabs tab;
     CB_TRY(tables(c, (long long)nmax, &tab, n2 > 0));
     // pairs whose rows the one-degree kernel forms again (GridGeo::npole)
-    const int npole = n2 > 0 && kgrad > 0 ? G.npole : 0;
+    const int npole = n2 > 0 && (kgrad > 0 || dlat > 0) ? G.npole : 0;
     // some latitudes on the one-degree path
-    const bool old_too = n2 < np || npole > 0;
+    const bool old_too = n2 < np || (npole > 0 && kgrad > 0);
     // Host coefficients of a call whose grid goes to the host are uploaded
     // later, in bands of orders overlapped with the synthesis of the first
     // band of latitudes (when the call runs in bands), else all now.
@@ -1907,6 +1907,13 @@ Status shs_grid_run(Context &c, const charm_point *pnt, const CoefIn &in,
     if (n2 > 0)
         CB_TRY(dbuf(c, "two_cs", (size_t)(2 * two_steps((long long)nmax)) *
                                      fam.nfam, &dcs2));
+    // what the rows at a pole read: C, S themselves, which the gradients'
+    // families begin with; those of a latitudinal derivative lack them or
+    // carry the factors of a radial one
+    double2 *dpole = dcs;
+    if (npole > 0 && kgrad == 0)
+        CB_TRY(dbuf(c, "two_cs_pole", (size_t)((nmax + 1) * (nmax + 2) / 2),
+                    &dpole));
     if (!in.dc)
     {
         CB_TRY(dbuf(c, "shc_in", (size_t)(2 * Ts), &raw));
@@ -1933,6 +1940,12 @@ Status shs_grid_run(Context &c, const charm_point *pnt, const CoefIn &in,
                                  c.stream), s2);
         if (with)
             G.pending = false;
+        if (dpole != dcs)
+        {
+            S.cs = dpole;
+            S.cs2 = nullptr;
+            CB_CUDA(launch_two_scale(S, m_lo, m_hi, nullptr, c.stream), s2);
+        }
         return s2;
     };
     auto all_coefs = [&]() -> Status {
@@ -2052,8 +2065,8 @@ Status shs_grid_run(Context &c, const charm_point *pnt, const CoefIn &in,
                 launch_shs_two(b, K, blocks(b.nitems), c.stream);
             if (e != cudaSuccess || p0 > 0 || npole == 0)
                 return e;
-            // (the families' first one-degree form is C, S themselves)
             ShsGridArgs a = A;
+            a.cs = dpole;
             a.npairs = npole;
             a.ntiles = (npole + 31) / 32;
             a.m0 = m_lo;
