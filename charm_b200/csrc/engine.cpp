@@ -1395,8 +1395,9 @@ bool shs_k_settled(Context &c, int kgrad, int dr, int dlat, int variant,
     return c.tuned.count(key) > 0 || !autotune_on() || nmax < 256;
 }
 
-// launch(K) runs the call's synthesis with K pairs per lane (its counter
-// cleared); cands: the widths to time, besides the built-in *K.
+// launch(K, work) runs the call's synthesis with K pairs per lane (its counter
+// cleared), with work = false over no orders; cands: the widths to time, one of
+// them to be taken as it is.
 template <typename F>
 Status tune_shs_k(Context &c, const F &launch, std::vector<int> cands,
                   int kgrad, int dr, int dlat, int variant, long long nmax,
@@ -1412,23 +1413,31 @@ Status tune_shs_k(Context &c, const F &launch, std::vector<int> cands,
     }
     if (!autotune_on() || nmax < 256)
         return st;
+    if (cands.size() == 1)
+    {
+        c.tuned[key].first = *K = cands[0];
+        return st;
+    }
     cudaEvent_t e0 = ev_get(c), e1 = ev_get(c);
     std::vector<std::pair<int, float>> meas;
     int best = *K;
     float best_ms = 0.0f;
-    // every candidate runs once untimed: a kernel's first launch in a process
-    // loads its code (about 40 us, more than some of these launches take)
+    // a kernel's first launch in a process loads its code (about 40 us, more
+    // than some of these launches take): a launch without work each, then one
+    // for the caches, then one timed
     for (int k : cands)
-        CB_CUDA(launch(k), st);
+        CB_CUDA(launch(k, false), st);
+    CB_CUDA(launch(*K, true), st);
+    c.launches += cands.size() + 1;
     for (int k : cands)
     {
         CB_CUDA(cudaEventRecord(e0, c.stream), st);
-        CB_CUDA(launch(k), st);
+        CB_CUDA(launch(k, true), st);
         CB_CUDA(cudaEventRecord(e1, c.stream), st);
         CB_CUDA(cudaEventSynchronize(e1), st);
         float ms = 0.0f;
         CB_CUDA(cudaEventElapsedTime(&ms, e0, e1), st);
-        c.launches += 2;
+        c.launches++;
         meas.emplace_back(k, ms);
         if (best_ms == 0.0f || ms < best_ms)
         {
@@ -2087,21 +2096,26 @@ Status shs_grid_run(Context &c, const charm_point *pnt, const CoefIn &in,
     int K = n2 > 0 ? choose_k_two(n2, mode) : choose_k(kgrad, dlat, np);
     // autotuned tile (first call of this shape)
     {
-        auto trial = [&](int k) {
+        auto trial = [&](int k, bool work) {
             const cudaError_t e = cudaMemsetAsync(
                 G.counter, 0, 17 * sizeof(unsigned long long), c.stream);
-            return e != cudaSuccess ? e
-                                    : synth(k, 0, np, 0, (long long)nmax + 1,
-                                            G.counter);
+            return e != cudaSuccess
+                       ? e
+                       : synth(k, 0, np, 0, work ? (long long)nmax + 1 : 0,
+                               G.counter);
         };
         const bool timed = !shs_k_settled(c, kgrad, dr, dlat, variant,
                                           (long long)nmax, np);
         std::vector<int> cands =
             kgrad >= 1 || dlat > 0 ? std::vector<int>{1, 2}
                                    : std::vector<int>{1, 2, 4};
+        // (of the widths 1..8 at 1..1801 pairs, nmax 400..3600, 1 was the
+        // fastest up to 64 pairs, 1 or 2 below 700, 3, 4 or 5 above, within
+        // 1%; each width timed is one more launch of a shape's first call)
         if (n2 > 0 && mode == 0)
-            cands = n2 <= 1024 ? std::vector<int>{1, 2, 3, 4, 5, 6}
-                               : std::vector<int>{3, 4, 5, 6, 7, 8};
+            cands = n2 <= 64    ? std::vector<int>{1}
+                    : n2 < 700 ? std::vector<int>{1, 2}
+                               : std::vector<int>{3, 4, 5};
         CB_TRY(tune_shs_k(c, trial, cands, kgrad, dr, dlat, variant,
                           (long long)nmax, np, &K));
         if (timed)

@@ -91,7 +91,7 @@ static_assert(near_stage(5) >= two_stage(5), "the larger stage sets the size");
 constexpr int two_min_blocks(int nf, int K)
 {
     if (nf == 1)
-        return K >= 7 ? 2 : (K >= 5 ? 3 : 4);
+        return K >= 5 ? 3 : 4;
     return nf * K >= 8 ? 2 : (nf * K >= 5 ? 3 : 4);
 }
 
@@ -688,8 +688,6 @@ static cudaError_t launch_mode(const ShsTwoArgs &A, int K, int grid,
     {
         switch (K)
         {
-        case 8: return launch_one<MODE, 8>(A, grid, st);
-        case 7: return launch_one<MODE, 7>(A, grid, st);
         case 6: return launch_one<MODE, 6>(A, grid, st);
         case 5: return launch_one<MODE, 5>(A, grid, st);
         case 4: return launch_one<MODE, 4>(A, grid, st);
