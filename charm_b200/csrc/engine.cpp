@@ -1616,6 +1616,12 @@ Status geometry_launch(Context &c, GridGeo *G)
 // form of the coefficients).
 constexpr unsigned long TWO_MIN_NMAX = 128;
 constexpr unsigned long TWO_MIN_NMAX_ONE = 400;
+// and from more pairs than one warp on: with fewer, the second form of the
+// coefficients (and the powers of a radius ratio) cost more than the shorter
+// columns give.  Call of nine latitudes above the sphere at nmax 1440, 2190:
+// 112 and 185 us with both, 97 and 159 without; of 33: 124 and 188, 132 and
+// 226 by the one-degree kernel alone.
+constexpr int TWO_MIN_PAIRS_ONE = 33;
 // The same for the analysis, whose transpose-reduce weighs more the shorter
 // the columns are: degree and evaluated pairs (GL nmax 520, 700, 850: 53,
 // 72, 98 us against 44, 76, 119 with the one-degree kernel, and about 5 us
@@ -1625,12 +1631,12 @@ constexpr int TWO_MIN_PAIRS_SHA = 384;
 constexpr double POLE_COS = 1e-6;
 
 // weights (analysis): the rows' quadrature weights times cw are uploaded too.
-// r_eq: every row at the coefficients' radius R (nothing to fold); two_min:
-// the least degree for the two-degree recurrence.
+// r_eq: every row at the coefficients' radius R (nothing to fold); two_min,
+// two_np: the least degree and number of pairs for the two-degree recurrence.
 Status grid_geometry(Context &c, const charm_point *pnt, const Pairs &P,
                      unsigned long nmax, double R, bool r_eq,
-                     unsigned long two_min, double cw, bool weights,
-                     GridGeo *G)
+                     unsigned long two_min, int two_np, double cw,
+                     bool weights, GridGeo *G)
 {
     Status st;
     const int np = (int)P.row_n.size();
@@ -1664,11 +1670,12 @@ Status grid_geometry(Context &c, const charm_point *pnt, const Pairs &P,
         hrs[p] = rs;
     }
     // folding keeps every power within the range of a double with room for
-    // the chunk scaling of the one-degree tables
+    // the chunk scaling of the one-degree tables, and pays (the powers are a
+    // launch of their own) where there are enough pairs
     if (!weights && !r_eq)
     {
         const double rho = R / r0;
-        G->rr = !(uniform && std::fabs(std::log2(rho)) *
+        G->rr = !(uniform && np >= two_np && std::fabs(std::log2(rho)) *
                                      (double)(nmax + 3) <= 600.0);
         if (!G->rr)
         {
@@ -1677,8 +1684,7 @@ Status grid_geometry(Context &c, const charm_point *pnt, const Pairs &P,
         }
     }
     const bool range = latitudes_in_range(hlat, np);
-    if (!G->rr && range && nmax >= two_min && !c.one_degree &&
-        (!weights || np >= TWO_MIN_PAIRS_SHA))
+    if (!G->rr && range && nmax >= two_min && np >= two_np && !c.one_degree)
         G->n2 = two_pairs(hlat, np, &G->polar);
     c.two_live = G->n2 > 0;
     // nothing for k_geometry to do but the sines: they come from the host
@@ -1881,10 +1887,10 @@ Status shs_grid_run(Context &c, const charm_point *pnt, const CoefIn &in,
     mur_dorder(in.mu, in.r, kgrad, dr, dlat, dlon, &mur, &dorder, &npar);
 
     GridGeo G;
+    const bool one = kgrad == 0 && dlat == 0;
     CB_TRY(grid_geometry(c, pnt, P, nmax, in.r, r_eq,
-                         kgrad > 0 || dlat > 0 ? TWO_MIN_NMAX
-                                               : TWO_MIN_NMAX_ONE,
-                         0.0, false, &G));
+                         one ? TWO_MIN_NMAX_ONE : TWO_MIN_NMAX,
+                         one ? TWO_MIN_PAIRS_ONE : 1, 0.0, false, &G));
     // ShsTwoArgs::mode and its coefficient families
     const int mode = kgrad == 0 ? dlat : 2 + kgrad;
     ScaleArgs fam{};
@@ -2550,8 +2556,8 @@ Status shs_batch_run(Context &c, const charm_point *pnt, size_t nsets,
     CB_TRY(batch_pairs(c, pnt, N, R, &BG));
     const int np = BG.np;
     GridGeo G;
-    CB_TRY(grid_geometry(c, pnt, BG.P, N, R, BG.r_eq, TWO_MIN_NMAX, 0.0, false,
-                         &G));
+    CB_TRY(grid_geometry(c, pnt, BG.P, N, R, BG.r_eq, TWO_MIN_NMAX, 1, 0.0,
+                         false, &G));
     const int n2 = G.n2;
     const bool two = n2 > 0;
     const int npole = two && kgrad > 0 ? G.npole : 0;
@@ -3535,8 +3541,8 @@ Status sha_grid_run(Context &c, const charm_point *pnt, const double *f_host,
     }
     const int np = (int)P.row_n.size();
     GridGeo G;
-    CB_TRY(grid_geometry(c, pnt, P, nmax, R, true, TWO_MIN_NMAX_SHA, cq, true,
-                         &G));
+    CB_TRY(grid_geometry(c, pnt, P, nmax, R, true, TWO_MIN_NMAX_SHA,
+                         TWO_MIN_PAIRS_SHA, cq, true, &G));
     const int n2 = G.n2;
     unsigned *const d_status = G.d_status;
 
