@@ -70,30 +70,30 @@ __global__ void RFFT_BOUNDS(NR) k_rfft_inv4(RfftArgs A)
 {
     extern __shared__ __align__(16) double2 s[];
     const int tid = threadIdx.x;
-    pick_rows(A);
+    const RfftRows R = pick_rows<true>(A);
     const long long row = blockIdx.x >> 1;
     const int rho = (int)(blockIdx.x & 1);
-    SrcQuarter src{A.X + row * A.ldX, A.w, A.w4, A.H, A.kmax, rho};
+    SrcQuarter src{R.X + row * A.ldX, A.w, A.w4, A.H, R.kmax, rho};
     fft_ct<MC, 0, true>(s, A.tw, tid, src, A.bh);
     fft_ct<MC, 0, false, ct_npass(MC) - 1>(s, A.tw, tid, SrcSmem{s},
                                               nullptr);
     fft_ct_last_out<MC>(
         s, A.tw, tid, A.H,
-        OutRowQ{reinterpret_cast<double2 *>(A.x + row * A.ldx), A.w, rho});
+        OutRowQ{reinterpret_cast<double2 *>(R.x + row * A.ldx), A.w, rho});
 }
 
 // Synthesis of rows of odd length L = H: Bluestein over the whole row
 // (run-time plan), the row being the real part of the inverse DFT.
-template <int V, int NR>
+template <int V, int NR, bool BATCH>
 __global__ void RFFT_BOUNDS(NR) k_rfft_inv_odd(RfftArgs A)
 {
     extern __shared__ __align__(16) double2 s[];
     const int tid = threadIdx.x, T = blockDim.x;
-    pick_rows(A);
+    const RfftRows R = pick_rows<BATCH>(A);
     const long long row = blockIdx.x;
-    SrcSpectrumOdd src{A.X + row * A.ldX, A.w, A.H, A.kmax};
+    SrcSpectrumOdd src{R.X + row * A.ldX, A.w, A.H, R.kmax};
     dft_h<V, 0>(s, A, tid, T, src);
-    double *x = A.x + row * A.ldx;
+    double *x = R.x + row * A.ldx;
     for (int j = tid; j < A.H; j += T)
         x[j] = dft_h_out(s, A, j).x;
 }
@@ -146,7 +146,7 @@ __global__ void RFFT_BOUNDS(NR) k_rfftc_fwd(RfftArgs A)
 
 // Synthesis direction of a cluster plan: rows of even length (ODD false,
 // pairs x_2t + i x_2t+1 for t < H) or of odd length H (the real part).
-template <int V, int NR, bool ODD, int MC = 0>
+template <int V, int NR, bool ODD, int MC, bool BATCH>
 __global__ void RFFT_BOUNDS(NR) k_rfftc_inv(RfftArgs A)
 {
     namespace cg = cooperative_groups;
@@ -155,17 +155,17 @@ __global__ void RFFT_BOUNDS(NR) k_rfftc_inv(RfftArgs A)
     const int tid = threadIdx.x, T = blockDim.x;
     const int C = A.C, q = (int)cl.block_rank(), H = A.H;
     const int Mc = A.M / C;
-    pick_rows(A);
+    const RfftRows R = pick_rows<BATCH>(A);
     const long long row = blockIdx.x / C;
     if constexpr (ODD)
     {
-        SrcSpectrumOdd src{A.X + row * A.ldX, A.w, H, A.kmax};
+        SrcSpectrumOdd src{R.X + row * A.ldX, A.w, H, R.kmax};
         SrcClusterDif<SrcSpectrumOdd> dif{src, A.twM, q, C, Mc, A.M, H};
         fft_m<V>(s, A.tw, Mc, A.npass, tid, T, dif, A.bh + (size_t)q * Mc);
     }
     else
     {
-        SrcSpectrum src{A.X + row * A.ldX, A.w, A.ht, H, A.kmax};
+        SrcSpectrum src{R.X + row * A.ldX, A.w, A.ht, H, R.kmax};
         SrcClusterDif<SrcSpectrum> dif{src, A.twM, q, C, Mc, A.M, H};
         if constexpr (MC > 0)
             fft_ct<MC, 0, false>(s, A.tw, tid, dif,
@@ -186,9 +186,9 @@ __global__ void RFFT_BOUNDS(NR) k_rfftc_inv(RfftArgs A)
         const double2 v = cluster_v(cl, s, A.twM, C, Mc, A.M, t);
         const double2 z = cmul(__ldg(&A.w[t]), conj2(v));
         if constexpr (ODD)
-            A.x[row * A.ldx + t] = z.x;
+            R.x[row * A.ldx + t] = z.x;
         else
-            reinterpret_cast<double2 *>(A.x + row * A.ldx)[t] = conj2(z);
+            reinterpret_cast<double2 *>(R.x + row * A.ldx)[t] = conj2(z);
     }
     cl.sync();
 }
@@ -310,17 +310,22 @@ cudaError_t rfft_set_smem(size_t smem)
 {
     const void *fns[] = {
         (const void *)k_rfft_fwd<false, 0>,
-        (const void *)k_rfft_inv<false, 0>,
+        (const void *)k_rfft_inv<false, 0, false>,
+        (const void *)k_rfft_inv<false, 0, true>,
         (const void *)k_rfft_fwd<true, 0>,
-        (const void *)k_rfft_inv<true, 0>,
+        (const void *)k_rfft_inv<true, 0, false>,
         (const void *)k_rfft_inv4<16, 96, 4608>,
         (const void *)k_rfft_kernel_spectrum<16, 96>,
-        (const void *)k_rfft_inv_odd<16, 96>,
+        (const void *)k_rfft_inv_odd<16, 96, false>,
+        (const void *)k_rfft_inv_odd<16, 96, true>,
         (const void *)k_rfftc_fwd<16, 96>,
-        (const void *)k_rfftc_inv<16, 96, false>,
-        (const void *)k_rfftc_inv<16, 96, true>,
+        (const void *)k_rfftc_inv<16, 96, false, 0, false>,
+        (const void *)k_rfftc_inv<16, 96, false, 0, true>,
+        (const void *)k_rfftc_inv<16, 96, true, 0, false>,
+        (const void *)k_rfftc_inv<16, 96, true, 0, true>,
         (const void *)k_rfftc_fwd<16, 96, 6144>,
-        (const void *)k_rfftc_inv<16, 96, false, 6144>,
+        (const void *)k_rfftc_inv<16, 96, false, 6144, false>,
+        (const void *)k_rfftc_inv<16, 96, false, 6144, true>,
         (const void *)k_rfftc_kspec<16, 96>};
     for (const void *f : fns)
     {
@@ -331,10 +336,13 @@ cudaError_t rfft_set_smem(size_t smem)
     }
     // clusters of 16 CTAs (rows beyond 8 x 9216) are a non-portable size
     const void *cfns[] = {(const void *)k_rfftc_fwd<16, 96>,
-                          (const void *)k_rfftc_inv<16, 96, false>,
-                          (const void *)k_rfftc_inv<16, 96, true>,
+                          (const void *)k_rfftc_inv<16, 96, false, 0, false>,
+                          (const void *)k_rfftc_inv<16, 96, false, 0, true>,
+                          (const void *)k_rfftc_inv<16, 96, true, 0, false>,
+                          (const void *)k_rfftc_inv<16, 96, true, 0, true>,
                           (const void *)k_rfftc_fwd<16, 96, 6144>,
-                          (const void *)k_rfftc_inv<16, 96, false, 6144>};
+                          (const void *)k_rfftc_inv<16, 96, false, 6144, false>,
+                          (const void *)k_rfftc_inv<16, 96, false, 6144, true>};
     for (const void *f : cfns)
     {
         // where refused, plans with 16 CTAs fail their occupancy check
@@ -368,8 +376,8 @@ int rfftc_max_clusters(int C, int Mc)
         return 0;
     }
     int n2 = 0;
-    if (cudaOccupancyMaxActiveClusters(&n2, k_rfftc_inv<16, 96, false>,
-                                       &cfg) != cudaSuccess)
+    if (cudaOccupancyMaxActiveClusters(
+            &n2, k_rfftc_inv<16, 96, false, 0, false>, &cfg) != cudaSuccess)
     {
         cudaGetLastError();
         return 0;
@@ -445,11 +453,16 @@ cudaError_t launch_rfft(const RfftArgs &A, bool inverse, cudaStream_t st)
         if (!inverse)
             return ct ? cudaLaunchKernelEx(&cfg, k_rfftc_fwd<16, 96, 6144>, A)
                       : cudaLaunchKernelEx(&cfg, k_rfftc_fwd<16, 96>, A);
-        if (A.odd)
-            return cudaLaunchKernelEx(&cfg, k_rfftc_inv<16, 96, true>, A);
-        return ct ? cudaLaunchKernelEx(&cfg, k_rfftc_inv<16, 96, false, 6144>,
-                                       A)
-                  : cudaLaunchKernelEx(&cfg, k_rfftc_inv<16, 96, false>, A);
+        void (*const fn[2][3])(RfftArgs) = {
+            {k_rfftc_inv<16, 96, false, 0, false>,
+             k_rfftc_inv<16, 96, false, 6144, false>,
+             k_rfftc_inv<16, 96, true, 0, false>},
+            {k_rfftc_inv<16, 96, false, 0, true>,
+             k_rfftc_inv<16, 96, false, 6144, true>,
+             k_rfftc_inv<16, 96, true, 0, true>}};
+        return cudaLaunchKernelEx(&cfg,
+                                  fn[A.batch ? 1 : 0][A.odd ? 2 : ct ? 1 : 0],
+                                  A);
     }
     const size_t smem = rfft_smem_bytes(A.M);
     const int T = A.M / 16;
@@ -458,7 +471,10 @@ cudaError_t launch_rfft(const RfftArgs &A, bool inverse, cudaStream_t st)
         // rows of odd length: synthesis only, Bluestein, run-time plan
         if (!inverse || A.f32_rows || A.direct)
             return cudaErrorInvalidValue;
-        k_rfft_inv_odd<16, 96><<<dim3(grid, ny), T, smem, st>>>(A);
+        if (A.batch)
+            k_rfft_inv_odd<16, 96, true><<<dim3(grid, ny), T, smem, st>>>(A);
+        else
+            k_rfft_inv_odd<16, 96, false><<<grid, T, smem, st>>>(A);
         return cudaGetLastError();
     }
     if (A.quarter)
@@ -487,15 +503,19 @@ cudaError_t launch_rfft(const RfftArgs &A, bool inverse, cudaStream_t st)
     const dim3 g2(grid, ny);
     if (A.f32_rows)
     {
+        if (A.batch)
+            return cudaErrorInvalidValue;
         if (inverse)
-            k_rfft_inv<true, 0><<<g2, T, smem, st>>>(A);
+            k_rfft_inv<true, 0, false><<<grid, T, smem, st>>>(A);
         else
-            k_rfft_fwd<true, 0><<<g2, T, smem, st>>>(A);
+            k_rfft_fwd<true, 0><<<grid, T, smem, st>>>(A);
     }
+    else if (inverse && A.batch)
+        k_rfft_inv<false, 0, true><<<g2, T, smem, st>>>(A);
     else if (inverse)
-        k_rfft_inv<false, 0><<<g2, T, smem, st>>>(A);
+        k_rfft_inv<false, 0, false><<<grid, T, smem, st>>>(A);
     else
-        k_rfft_fwd<false, 0><<<g2, T, smem, st>>>(A);
+        k_rfft_fwd<false, 0><<<grid, T, smem, st>>>(A);
     return cudaGetLastError();
 }
 

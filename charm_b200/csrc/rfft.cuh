@@ -902,16 +902,17 @@ constexpr int RFFT_NR = 96;
 #define RFFT_BOUNDS(NR) __maxnreg__(NR)
 
 // This CTA's part of a launch: rows of one batch entry (blockIdx.y), or of A
-// itself.
-__device__ __forceinline__ void pick_rows(RfftArgs &A)
+// itself.  BATCH = false compiles the former out: with it the run-time plans
+// spill 520 bytes a thread (rows of GL nmax 767 23 us in the place of 19, of
+// nmax 1151 56 in the place of 47, 90 rows of 3001 points 43 in the place of
+// 37), so a launch without a batch has kernels of its own there.
+template <bool BATCH>
+__device__ __forceinline__ RfftRows pick_rows(const RfftArgs &A)
 {
-    if (A.batch)
-    {
-        const RfftRows b = A.batch[blockIdx.y];
-        A.x = b.x;
-        A.X = const_cast<double2 *>(b.X);
-        A.kmax = b.kmax;
-    }
+    if constexpr (BATCH)
+        if (A.batch)
+            return A.batch[blockIdx.y];
+    return {A.x, A.X, A.kmax};
 }
 
 // Analysis direction: real rows x[row][0..L) -> X[row][0..kmax]; one CTA
@@ -929,7 +930,7 @@ __global__ void RFFT_BOUNDS(RFFT_NR) k_rfft_fwd(RfftArgs A)
     const int H = A.H;
     // rows beyond the last are transformed again and not stored
     long long row = (long long)blockIdx.x * RP + sub;
-    const bool mine = row < A.nrows;
+    const bool mine = RP == 1 || row < A.nrows;
     if (!mine)
         row = A.nrows - 1;
     if constexpr (F32)
@@ -979,7 +980,7 @@ struct OutRow
     }
 };
 
-template <bool F32, int MC>
+template <bool F32, int MC, bool BATCH = true>
 __global__ void RFFT_BOUNDS(RFFT_NR) k_rfft_inv(RfftArgs A)
 {
     extern __shared__ __align__(16) double2 smem[];
@@ -988,21 +989,21 @@ __global__ void RFFT_BOUNDS(RFFT_NR) k_rfft_inv(RfftArgs A)
     const int sub = RP > 1 ? (int)threadIdx.x / T : 0;
     const int tid = (int)threadIdx.x - sub * T;
     double2 *s = smem + sub * (MC + MC / 8);
-    pick_rows(A);
+    const RfftRows R = pick_rows<BATCH>(A);
     long long row = (long long)blockIdx.x * RP + sub;
-    const bool mine = row < A.nrows;
+    const bool mine = RP == 1 || row < A.nrows;
     if (!mine)
         row = A.nrows - 1;
-    SrcSpectrum src{A.X + row * A.ldX, A.direct ? nullptr : A.w, A.ht, A.H,
-                    A.kmax};
+    SrcSpectrum src{R.X + row * A.ldX, A.direct ? nullptr : A.w, A.ht, A.H,
+                    R.kmax};
     bool done = false;
     if constexpr (MC > 0)
     if (!A.direct)
     {
         // Bluestein with the second FFT's last pass writing the row
-        void *x2 = F32 ? (void *)(reinterpret_cast<float *>(A.x) +
+        void *x2 = F32 ? (void *)(reinterpret_cast<float *>(R.x) +
                                   row * A.ldx)
-                       : (void *)(A.x + row * A.ldx);
+                       : (void *)(R.x + row * A.ldx);
         fft_ct<MC, 0, true>(s, A.tw, tid, src, A.bh);
         fft_ct<MC, 0, false, ct_npass(MC) - 1>(s, A.tw, tid, SrcSmem{s},
                                                nullptr);
@@ -1017,7 +1018,7 @@ __global__ void RFFT_BOUNDS(RFFT_NR) k_rfft_inv(RfftArgs A)
         return;
     if constexpr (F32)
     {
-        float *xf = reinterpret_cast<float *>(A.x);
+        float *xf = reinterpret_cast<float *>(R.x);
         float2 *x2 = reinterpret_cast<float2 *>(xf + row * A.ldx);
         for (int j = tid; j < A.H; j += T)
         {
@@ -1027,7 +1028,7 @@ __global__ void RFFT_BOUNDS(RFFT_NR) k_rfft_inv(RfftArgs A)
     }
     else
     {
-        double2 *x2 = reinterpret_cast<double2 *>(A.x + row * A.ldx);
+        double2 *x2 = reinterpret_cast<double2 *>(R.x + row * A.ldx);
         for (int j = tid; j < A.H; j += T)
             x2[j] = conj2(dft_h_out(s, A, j));
     }
