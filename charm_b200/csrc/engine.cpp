@@ -1617,11 +1617,19 @@ Status geometry_launch(Context &c, GridGeo *G)
 constexpr unsigned long TWO_MIN_NMAX = 128;
 constexpr unsigned long TWO_MIN_NMAX_ONE = 400;
 // and from more pairs than one warp on: with fewer, the second form of the
-// coefficients (and the powers of a radius ratio) cost more than the shorter
-// columns give.  Call of nine latitudes above the sphere at nmax 1440, 2190:
-// 112 and 185 us with both, 97 and 159 without; of 33: 124 and 188, 132 and
-// 226 by the one-degree kernel alone.
+// coefficients costs more than the shorter columns give (call of seventeen
+// pairs at nmax 1440 and 2190: 123 and 186 us against 93 and 152).  Grids with
+// pairs next to the equator need both forms: from 129 pairs (two- against
+// one-degree, mirror rows: 64 pairs at nmax 720, 1440, 3000 72, 124, 358 us
+// against 62, 114, 322; 128 pairs 74, 144, 454 against 77, 149, 457).
 constexpr int TWO_MIN_PAIRS_ONE = 33;
+constexpr int TWO_MIN_PAIRS_NEAR = 129;
+// One potential folds the ratio of the radii into the coefficients (whose
+// powers are a launch of their own, about 8 us) where degree times pairs
+// reaches this, else the rows keep their radius and the one-degree kernel: 64
+// and 128 pairs at nmax 500 60 and 64 us folded, 53 and 61 not, 65 pairs at
+// nmax 1440 119 and 149, 33 at 2190 187 and 212.
+constexpr long long TWO_MIN_FOLD = 70000;
 // The same for the analysis, whose transpose-reduce weighs more the shorter
 // the columns are: degree and evaluated pairs (GL nmax 520, 700, 850: 53,
 // 72, 98 us against 44, 76, 119 with the one-degree kernel, and about 5 us
@@ -1631,12 +1639,13 @@ constexpr int TWO_MIN_PAIRS_SHA = 384;
 constexpr double POLE_COS = 1e-6;
 
 // weights (analysis): the rows' quadrature weights times cw are uploaded too.
-// r_eq: every row at the coefficients' radius R (nothing to fold); two_min,
-// two_np: the least degree and number of pairs for the two-degree recurrence.
+// r_eq: every row at the coefficients' radius R (nothing to fold); two_min: the
+// least degree for the two-degree recurrence; one: a synthesis of one potential
+// or radial derivative of one set, which weighs its preparation.
 Status grid_geometry(Context &c, const charm_point *pnt, const Pairs &P,
                      unsigned long nmax, double R, bool r_eq,
-                     unsigned long two_min, int two_np, double cw,
-                     bool weights, GridGeo *G)
+                     unsigned long two_min, bool one, double cw, bool weights,
+                     GridGeo *G)
 {
     Status st;
     const int np = (int)P.row_n.size();
@@ -1675,8 +1684,9 @@ Status grid_geometry(Context &c, const charm_point *pnt, const Pairs &P,
     if (!weights && !r_eq)
     {
         const double rho = R / r0;
-        G->rr = !(uniform && np >= two_np && std::fabs(std::log2(rho)) *
-                                     (double)(nmax + 3) <= 600.0);
+        G->rr = !(uniform &&
+                  (!one || (long long)nmax * np >= TWO_MIN_FOLD) &&
+                  std::fabs(std::log2(rho)) * (double)(nmax + 3) <= 600.0);
         if (!G->rr)
         {
             G->rho = rho;
@@ -1684,8 +1694,12 @@ Status grid_geometry(Context &c, const charm_point *pnt, const Pairs &P,
         }
     }
     const bool range = latitudes_in_range(hlat, np);
+    const int two_np =
+        weights ? TWO_MIN_PAIRS_SHA : (one ? TWO_MIN_PAIRS_ONE : 1);
     if (!G->rr && range && nmax >= two_min && np >= two_np && !c.one_degree)
         G->n2 = two_pairs(hlat, np, &G->polar);
+    if (one && G->n2 < np && np < TWO_MIN_PAIRS_NEAR)
+        G->n2 = G->polar = 0;
     c.two_live = G->n2 > 0;
     // nothing for k_geometry to do but the sines: they come from the host
     // (and for the pairs at a pole in any case, so that their noise is the
@@ -1889,8 +1903,8 @@ Status shs_grid_run(Context &c, const charm_point *pnt, const CoefIn &in,
     GridGeo G;
     const bool one = kgrad == 0 && dlat == 0;
     CB_TRY(grid_geometry(c, pnt, P, nmax, in.r, r_eq,
-                         one ? TWO_MIN_NMAX_ONE : TWO_MIN_NMAX,
-                         one ? TWO_MIN_PAIRS_ONE : 1, 0.0, false, &G));
+                         one ? TWO_MIN_NMAX_ONE : TWO_MIN_NMAX, one, 0.0,
+                         false, &G));
     // ShsTwoArgs::mode and its coefficient families
     const int mode = kgrad == 0 ? dlat : 2 + kgrad;
     ScaleArgs fam{};
@@ -2556,8 +2570,8 @@ Status shs_batch_run(Context &c, const charm_point *pnt, size_t nsets,
     CB_TRY(batch_pairs(c, pnt, N, R, &BG));
     const int np = BG.np;
     GridGeo G;
-    CB_TRY(grid_geometry(c, pnt, BG.P, N, R, BG.r_eq, TWO_MIN_NMAX, 1, 0.0,
-                         false, &G));
+    CB_TRY(grid_geometry(c, pnt, BG.P, N, R, BG.r_eq, TWO_MIN_NMAX,
+                         false, 0.0, false, &G));
     const int n2 = G.n2;
     const bool two = n2 > 0;
     const int npole = two && kgrad > 0 ? G.npole : 0;
@@ -3541,8 +3555,8 @@ Status sha_grid_run(Context &c, const charm_point *pnt, const double *f_host,
     }
     const int np = (int)P.row_n.size();
     GridGeo G;
-    CB_TRY(grid_geometry(c, pnt, P, nmax, R, true, TWO_MIN_NMAX_SHA,
-                         TWO_MIN_PAIRS_SHA, cq, true, &G));
+    CB_TRY(grid_geometry(c, pnt, P, nmax, R, true, TWO_MIN_NMAX_SHA, false,
+                         cq, true, &G));
     const int n2 = G.n2;
     unsigned *const d_status = G.d_status;
 

@@ -1,6 +1,7 @@
-"""Grids of few latitudes either side of the 33 pairs from which the potential
-takes the two-degree recurrence and folds the rows' radius into the
-coefficients, against the CPU oracle.
+"""Grids of few latitudes either side of the lines from which the potential of
+one set takes the two-degree recurrence (33 pairs, 129 where some lie next to
+the equator, as they do here) and folds the rows' radius into the coefficients
+(degree times pairs 70000: 167 pairs), against the CPU oracle.
 
 Tolerance: both sides' functions of degree n carry about n 2^-53 of their size
 from the rounded latitude; 4 n 2^-53 in relative RMS over the rows, times 4 off
@@ -14,14 +15,15 @@ from oracle import orc
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("pairs", [1, 32, 33])
+@pytest.mark.parametrize("pairs", [1, 32, 33, 128, 129, 166, 167])
+@pytest.mark.parametrize("last", [0.02, 0.2])
 @pytest.mark.parametrize("mirror", [False, True])
 @pytest.mark.parametrize("ratio", [1.0, 1.02])
 @pytest.mark.parametrize("kind", [None, (1, 0, 0), (0, 0, 1)])
-def test_few_latitudes(pairs, mirror, ratio, kind):
+def test_few_latitudes(pairs, last, mirror, ratio, kind):
     import charm_b200 as cb
     n = 421
-    lat = np.linspace(1.3, 0.02, pairs)
+    lat = np.linspace(1.3, last, pairs)
     if mirror:
         lat = np.concatenate([lat, -lat[::-1]])
     lon = np.arange(2 * n + 2) * (np.pi / (n + 1))
