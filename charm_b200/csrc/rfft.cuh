@@ -666,12 +666,7 @@ __device__ __forceinline__ void dft_h(double2 *s, const RfftArgs &A, int tid,
 {
     if constexpr (MC > 0)
     {
-        // plan fixed at compile time (A.M == MC)
-        if (A.direct)
-        {
-            fft_ct<MC, 0, false>(s, A.tw, tid, pre, nullptr);
-            return;
-        }
+        // plan fixed at compile time (A.M == MC, Bluestein)
         fft_ct<MC, 0, true>(s, A.tw, tid, pre, A.bh);
         fft_ct<MC, 0, false, ct_npass(MC), true>(s, A.tw, tid, SrcSmem{s},
                                                     nullptr);
@@ -996,9 +991,7 @@ __global__ void RFFT_BOUNDS(RFFT_NR) k_rfft_inv(RfftArgs A)
         row = A.nrows - 1;
     SrcSpectrum src{R.X + row * A.ldX, A.direct ? nullptr : A.w, A.ht, A.H,
                     R.kmax};
-    bool done = false;
     if constexpr (MC > 0)
-    if (!A.direct)
     {
         // Bluestein with the second FFT's last pass writing the row
         void *x2 = F32 ? (void *)(reinterpret_cast<float *>(R.x) +
@@ -1009,31 +1002,28 @@ __global__ void RFFT_BOUNDS(RFFT_NR) k_rfft_inv(RfftArgs A)
                                                nullptr);
         fft_ct_last_out<MC>(s, A.tw, tid, mine ? A.H : 0,
                             OutRow<F32>{x2, A.w});
-        done = true;
-    }
-    if (done)
-        return;
-    dft_h<16, MC>(s, A, tid, T, src);
-    if (!mine)
-        return;
-    if constexpr (F32)
-    {
-        float *xf = reinterpret_cast<float *>(R.x);
-        float2 *x2 = reinterpret_cast<float2 *>(xf + row * A.ldx);
-        for (int j = tid; j < A.H; j += T)
-        {
-            const double2 z = conj2(dft_h_out(s, A, j));
-            x2[j] = make_float2((float)z.x, (float)z.y);
-        }
     }
     else
     {
-        double2 *x2 = reinterpret_cast<double2 *>(R.x + row * A.ldx);
-        for (int j = tid; j < A.H; j += T)
-            x2[j] = conj2(dft_h_out(s, A, j));
+        dft_h<16, 0>(s, A, tid, T, src);
+        if constexpr (F32)
+        {
+            float *xf = reinterpret_cast<float *>(R.x);
+            float2 *x2 = reinterpret_cast<float2 *>(xf + row * A.ldx);
+            for (int j = tid; j < A.H; j += T)
+            {
+                const double2 z = conj2(dft_h_out(s, A, j));
+                x2[j] = make_float2((float)z.x, (float)z.y);
+            }
+        }
+        else
+        {
+            double2 *x2 = reinterpret_cast<double2 *>(R.x + row * A.ldx);
+            for (int j = tid; j < A.H; j += T)
+                x2[j] = conj2(dft_h_out(s, A, j));
+        }
     }
 }
-
 
 // launch of the one-CTA kernels with the compile-time plan MC
 template <int MC>
