@@ -397,7 +397,8 @@ def run_ours(args):
     # execute fewer FP64 instructions per unit, reported as
     # fp64_instr_per_unit: 4 with the one-degree recurrence (1 DMUL + 1 DFMA,
     # even/odd lumped sums 2 DFMA), 3 with the two-degree one, which both
-    # directions take on a GL grid from 767 rows (384 pairs) on.
+    # directions take on a GL grid from 767 rows (384 pairs,
+    # TWO_MIN_PAIRS_SHA of the engine) on.
     P_pairs = (nlat + 1) // 2
     units = T * P_pairs
     shs_ms = ms[0] / max(cnt[0], 1)

@@ -731,10 +731,6 @@ void host_smm(long long nmax, double *smm)
     }
 }
 
-// Steps of the two-degree recurrence over all orders of degree nmax
-// (two_sum of two.cuh).
-long long two_steps(long long nmax) { return ((nmax + 2) * (nmax + 2)) / 4; }
-
 // Recurrence tables of the rescaled recurrence (leg.cuh, tables.cu), built
 // once per maximum degree and kept on the device.
 struct Tabs
@@ -783,7 +779,7 @@ Status tables(Context &c, long long nmax, Tabs *tab, bool two = false)
     }
     if (two)
     {
-        const size_t TL = (size_t)two_steps(nmax);
+        const size_t TL = (size_t)two_sum(nmax);
         CB_TRY(dbuf(c, "tab_ab" + sfx, TL, &tab->ab));
         CB_TRY(dbuf(c, "tab_ag" + sfx, TL, &tab->ag));
         CB_TRY(dbuf(c, "tab_kw" + sfx, 3 * TL, &tab->kw));
@@ -1749,7 +1745,7 @@ Status grid_geometry(Context &c, const charm_point *pnt, const Pairs &P,
     if (G->n2 > 0)
     {
         double2 *pw = nullptr;
-        A.npow = 64 + (int)(nmax / 64) + 1;   // pow_entries of two.cuh
+        A.npow = pow_entries((long long)nmax);
         CB_TRY(dbuf(c, "geo_pow", (size_t)A.npow * np, &pw));
         A.pw = pw;
         G->pw = pw;
@@ -1934,7 +1930,7 @@ Status shs_grid_run(Context &c, const charm_point *pnt, const CoefIn &in,
                     (size_t)((nmax + 1) * (nmax + 2) / 2) *
                         (n2 > 0 ? fam.nfam : 1), &dcs));
     if (n2 > 0)
-        CB_TRY(dbuf(c, "two_cs", (size_t)(2 * two_steps((long long)nmax)) *
+        CB_TRY(dbuf(c, "two_cs", (size_t)(2 * two_sum((long long)nmax)) *
                                      fam.nfam, &dcs2));
     // what the rows at a pole read: C, S themselves, which the gradients'
     // families begin with; those of a latitudinal derivative lack them or
@@ -2585,7 +2581,7 @@ Status shs_batch_run(Context &c, const charm_point *pnt, size_t nsets,
     CB_TRY(tables(c, (long long)N, &tab, n2 > 0));
     const long long T = (long long)(N + 1) * (N + 2) / 2 *
                         (two ? fam.nfam : 1);
-    const long long T2 = 2 * two_steps((long long)N) * fam.nfam;
+    const long long T2 = 2 * two_sum((long long)N) * fam.nfam;
     double2 *cs_all = nullptr, *cs2_all = nullptr;
     // the kernels' forms of set j's coefficients, at place k of the buffers
     auto scale = [&](size_t j, size_t k) -> Status {
@@ -3582,7 +3578,7 @@ Status sha_grid_run(Context &c, const charm_point *pnt, const double *f_host,
     Gn = (ntiles + tpg - 1) / tpg;
     double2 *part = nullptr, *part1 = nullptr;
     CB_TRY(dbuf(c, "sha_part",
-                (size_t)Gn * (n2 > 0 ? 2 * two_steps((long long)nmax) : T),
+                (size_t)Gn * (n2 > 0 ? 2 * two_sum((long long)nmax) : T),
                 &part));
     if (n2 > 0 && n2 < np)
         CB_TRY(dbuf(c, "sha_part1", (size_t)T, &part1));

@@ -16,6 +16,19 @@ enum : unsigned
                                  // the tensor-core synthesis
 };
 
+// Sizes of the two-degree recurrence's arrays (two.cuh).
+// steps of all orders whose nmax - m is 0 .. j
+__host__ __device__ __forceinline__ long long two_sum(long long j)
+{
+    return ((j + 2) * (j + 2)) / 4;
+}
+// entries of a latitude's power table (two_seed): u^r, r < POW_LOW, and
+// u^(POW_LOW j) up to degree nmax
+constexpr int POW_LOW = 64;
+__host__ __device__ __forceinline__ int pow_entries(long long nmax)
+{
+    return POW_LOW + (int)(nmax / POW_LOW) + 1;
+}
 
 // One coefficient set of a batched synthesis: its degree, its first work
 // item, its scaled coefficients (in the layout of the shared tables' degree)
@@ -136,7 +149,7 @@ struct GeometryArgs
 };
 
 // Coefficients of one set into the forms the grid syntheses read
-// (k_two_scale, k_scale_cs).
+// (k_two_scale).
 struct ScaleArgs
 {
     long long ntab;          // degree of the tables (layout of cs, cs2)
@@ -444,7 +457,6 @@ cudaError_t launch_tables(long long nmax, const double *r, const double *ri,
 cudaError_t launch_scale_cs(long long nmax, long long shc_nmax,
                             const double *c, const double *s,
                             const double *tc, double2 *cs, cudaStream_t st);
-// same into the layout of degree ntab >= nmax (zero above nmax)
 cudaError_t launch_shs_grid(const ShsGridArgs &A, int kgrad, int dr,
                             int dlat, bool rr, int K, int grid,
                             cudaStream_t st);

@@ -19,8 +19,9 @@
 //     and a second FFT_M (conjugated in and out, which inverts it);
 //   * FFT_M by in-place Stockham autosort passes (two to four of radix 3 to
 //     18 in the compile-time plans, CT_PLANS in rfft.cuh; radix 8, 4, 2 and
-//     3 in the run-time plans, which the kernel spectra, odd rows and the
-//     clusters without a fixed length use): every thread holds V values
+//     3 in the run-time plans, which direct transforms, M = 6144 in one CTA,
+//     odd rows, the kernel spectra and the clusters without a fixed length
+//     use): every thread holds V values
 //     across the barrier that separates the loads of a pass from its
 //     stores, so one buffer of M values suffices.  The first pass reads its
 //     inputs straight from global memory (with the chirp applied; the zero
@@ -486,7 +487,7 @@ cudaError_t launch_rfft(const RfftArgs &A, bool inverse, cudaStream_t st)
         k_rfft_inv4<16, 96, 4608><<<dim3(2 * grid, ny), T, smem, st>>>(A);
         return cudaGetLastError();
     }
-    // Bluestein: every length has its plan fixed at compile time
+    // Bluestein: the plans fixed at compile time, all lengths but 6144
     if (!A.direct)
     {
         static bool (*const group[])(const RfftArgs &, bool, cudaStream_t,

@@ -442,11 +442,13 @@ __device__ __forceinline__ void fft_m(double2 *s,
 // Radices, strides, thread counts and butterfly ranges become constants, so
 // the index arithmetic of every pass folds away, and the larger radices cut
 // the number of barrier-separated passes through shared memory (4608 = 16 16
-// 18: three passes instead of five).  Every length that Bluestein's algorithm
-// can ask of one CTA, 2^a 3^b with 6 <= a and at most 9216, has a plan.  The
-// first radix is 16 or 8 (the zero half of a chirped sequence is skipped
-// there), the last even (the half-output passes), and every pass keeps M / R
-// and the stride a multiple of 8 (the padded layout).
+// 18: three passes instead of five).  The lengths are those that Bluestein's
+// algorithm can ask of one CTA, 2^a 3^b with 6 <= a and at most 9216; 6144,
+// which ends in radix 3, serves the clusters alone (one CTA runs that length,
+// and the direct transforms, by the run-time plan).  The first radix is 16 or
+// 8 (the zero half of a chirped sequence is skipped there), the last of the
+// others even (the half-output passes), and every pass keeps M / R and the
+// stride a multiple of 8 (the padded layout).
 struct CtPlan
 {
     int M, n, r[4];

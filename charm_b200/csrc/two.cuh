@@ -34,6 +34,7 @@
 #pragma once
 
 #include "common.cuh"
+#include "kernels.h"
 #include "leg.cuh"
 
 namespace cb
@@ -46,12 +47,6 @@ __host__ __device__ __forceinline__ long long two_len(long long nmax,
                                                       long long m)
 {
     return (nmax - m) / 2 + 1;
-}
-
-// steps of all orders whose nmax - m is 0 .. j
-__host__ __device__ __forceinline__ long long two_sum(long long j)
-{
-    return ((j + 2) * (j + 2)) / 4;
 }
 
 // first step of order m in order-major arrays of degree nmax
@@ -68,13 +63,6 @@ __host__ __device__ __forceinline__ long long two_col0(long long nmax,
 // one product instead of the 2 log2(m) dependent ones of pow_me, which were
 // a third of the kernel's instructions at nmax 2190.
 // ---------------------------------------------------------------------------
-constexpr int POW_LOW = 64;
-
-__host__ __device__ __forceinline__ int pow_entries(long long nmax)
-{
-    return POW_LOW + (int)(nmax / POW_LOW) + 1;
-}
-
 // 2^e for -1022 <= e <= 1023
 __device__ __forceinline__ double pow2i(int e)
 {
@@ -82,9 +70,13 @@ __device__ __forceinline__ double pow2i(int e)
 }
 
 // Normalises a scaled state as leg_fixup does (true when the latitude turned
-// unscaled), with products by powers of two in place of scalbn: a chunk of
-// TWO_CHUNK steps multiplies the state by less than 2^330 (leg.cuh), so E is
-// above -1000 where it is used as an exponent.
+// unscaled), with products by powers of two in place of scalbn.  A chunk of
+// TWO_CHUNK steps multiplies the state by at most the 64 first factors
+// 1 / eps_m+i of its order, about ((2 m)^64 / 64!)^(1/2): 2^313 at m = 10800,
+// 2^402 at the largest order that the row transforms serve.  So a latitude
+// turns with E above -1000 up to m = 10800; beyond, where E is no exponent of
+// a double yet, it turns one chunk later (what it then leaves out is below
+// 2^-198).
 __device__ __forceinline__ bool two_fixup(double &x, double &y, int &E)
 {
     if (E == 0)

@@ -1,7 +1,7 @@
 """Forward modelling as one sequence of transforms whose status is read at its
 end: a Gauss--Legendre grid that fails in the middle (the limit of the Newton
-iterations lowered to one) is reported, leaves the caller's potential alone
-and is not kept for later calls."""
+iterations lowered to one) is reported and not kept for later calls; and a
+sequence of more stagings than there are slots."""
 import numpy as np
 import pytest
 
@@ -31,4 +31,26 @@ def test_failed_grid_is_reported_and_not_kept(monkeypatch):
     ref = orc.gfm_global(orc.Shc(N, 1.0, 1.0, c, s), N, R, None, None,
                          GRAV_CONST, MOON_MASS, 1, 2, top,
                          const_density=2600.0)
+    assert coef_rel_rms(pot.c, pot.s, ref.c, ref.s) <= 1e-12
+
+
+def test_more_transforms_than_staging_slots():
+    """Eighteen powers with three densities: 72 stagings (a synthesis of the
+    sets and three analyses a power) in one sequence of 64 slots."""
+    import charm_b200 as cb
+    R, N, top, powers = 1728000.0, 6, 20, 18
+    c, s = random_body(N, 5, R, 2000.0)
+    dens = []
+    for k in range(3):
+        dc, ds = random_body(4, 40 + k, 0.0, 30.0)
+        dc[0] = (2600.0, -2e-4, 1e-10)[k]
+        dens.append((4, dc, ds))
+    pot = cb.gfm_global_density_3d(
+        cb.Shc(N, 1.0, 1.0, c, s), N, R,
+        [cb.Shc(n, 1.0, 1.0, a, b) for n, a, b in dens], [4, 4, 4], 2,
+        GRAV_CONST, MOON_MASS, 1, powers, top)
+    ref = orc.gfm_global(
+        orc.Shc(N, 1.0, 1.0, c, s), N, R,
+        [orc.Shc(n, 1.0, 1.0, a, b) for n, a, b in dens], [4, 4, 4],
+        GRAV_CONST, MOON_MASS, 1, powers, top)
     assert coef_rel_rms(pot.c, pot.s, ref.c, ref.s) <= 1e-12
