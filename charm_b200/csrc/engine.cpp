@@ -304,13 +304,11 @@ Status init(Context &c)
 }
 
 // Frees what the two-degree recurrence keeps on the device (tables, its forms
-// of the coefficients, power tables, the equatorial sums): no call needs it
-// to be served.  True when there was any.
+// of the coefficients): no call needs it to be served.  True when there was
+// any.
 bool two_release(Context &c)
 {
-    static const char *const names[] = {"tab_ab", "tab_ag",   "tab_kw",
-                                        "tab_sm", "two_cs",   "two_batch_cs",
-                                        "geo_pow", "sha_part1"};
+    static const char *const names[] = {"tab_two", "two_cs", "two_batch_cs"};
     bool any = false;
     for (auto &kv : c.bufs)
         for (const char *n : names)
@@ -347,6 +345,11 @@ template <typename F> Status or_one_degree(Context &c, const F &call)
     } off{c};
     cudaStreamSynchronize(c.copy_stream);
     two_release(c);
+    // (with the equatorial sums behind it)
+    DevBuf &part = c.bufs["sha_part"];
+    cudaFree(part.p);
+    part = DevBuf{};
+    c.epoch++;
     c.one_degree = c.fell_back = true;
     return call();
 }
@@ -779,11 +782,13 @@ Status tables(Context &c, long long nmax, Tabs *tab, bool two = false)
     }
     if (two)
     {
+        // (one buffer: allocations are most of a new degree's first call)
         const size_t TL = (size_t)two_sum(nmax);
-        CB_TRY(dbuf(c, "tab_ab" + sfx, TL, &tab->ab));
-        CB_TRY(dbuf(c, "tab_ag" + sfx, TL, &tab->ag));
-        CB_TRY(dbuf(c, "tab_kw" + sfx, 3 * TL, &tab->kw));
-        CB_TRY(dbuf(c, "tab_sm" + sfx, (size_t)(nmax + 1), &tab->sm));
+        CB_TRY(dbuf(c, "tab_two" + sfx, 2 * TL + (3 * TL + nmax + 2) / 2,
+                    &tab->ab));
+        tab->ag = tab->ab + TL;
+        tab->kw = reinterpret_cast<double *>(tab->ag + TL);
+        tab->sm = tab->kw + 3 * TL;
     }
     auto build_two = [&]() -> Status {
         Status s2;
@@ -1708,7 +1713,11 @@ Status grid_geometry(Context &c, const charm_point *pnt, const Pairs &P,
     for (int p = 0; p < (plain ? np : given); p++)
         sincos(hlat[p], &ht[p], &hu[p]);
     void *dgeo = nullptr;
-    CB_TRY(buf(c, "geo", up + (size_t)np * 3 * 8, &dgeo));
+    // (behind the latitudes the power table of the two-degree recurrence)
+    const size_t geo_words = ((size_t)np * 7 + 1) / 2 * 2;
+    const int npow = G->n2 > 0 ? pow_entries((long long)nmax) : 0;
+    CB_TRY(buf(c, "geo", geo_words * 8 + (size_t)npow * np * sizeof(double2),
+               &dgeo));
     double *d = static_cast<double *>(dgeo);
     G->lat = d;
     G->rhos = G->w_n = d + np;
@@ -1742,14 +1751,9 @@ Status grid_geometry(Context &c, const charm_point *pnt, const Pairs &P,
     A.t = dt;
     A.u = dt + np;
     A.z = dt + 2 * np;
-    if (G->n2 > 0)
-    {
-        double2 *pw = nullptr;
-        A.npow = pow_entries((long long)nmax);
-        CB_TRY(dbuf(c, "geo_pow", (size_t)A.npow * np, &pw));
-        A.pw = pw;
-        G->pw = pw;
-    }
+    A.npow = npow;
+    if (npow > 0)
+        G->pw = A.pw = reinterpret_cast<double2 *>(d + geo_words);
     A.clear = static_cast<unsigned *>(sp);
     if (G->rho != 1.0)
     {
@@ -1925,20 +1929,23 @@ Status shs_grid_run(Context &c, const charm_point *pnt, const CoefIn &in,
     bool coef_later =
         !in.dc && !d_f &&
         shs_k_settled(c, kgrad, dr, dlat, variant, (long long)nmax, np);
-    if (old_too)
-        CB_TRY(dbuf(c, n2 > 0 ? "two_cs1" : "cs",
-                    (size_t)((nmax + 1) * (nmax + 2) / 2) *
-                        (n2 > 0 ? fam.nfam : 1), &dcs));
-    if (n2 > 0)
-        CB_TRY(dbuf(c, "two_cs", (size_t)(2 * two_sum((long long)nmax)) *
-                                     fam.nfam, &dcs2));
     // what the rows at a pole read: C, S themselves, which the gradients'
     // families begin with; those of a latitudinal derivative lack them or
     // carry the factors of a radial one
-    double2 *dpole = dcs;
-    if (npole > 0 && kgrad == 0)
-        CB_TRY(dbuf(c, "two_cs_pole", (size_t)((nmax + 1) * (nmax + 2) / 2),
-                    &dpole));
+    double2 *dpole = nullptr;
+    const size_t T1 = (size_t)((nmax + 1) * (nmax + 2) / 2);
+    if (n2 > 0)
+    {
+        const size_t T2 = (size_t)(2 * two_sum((long long)nmax)) * fam.nfam;
+        const size_t To = old_too ? T1 * fam.nfam : 0;
+        const bool own = npole > 0 && kgrad == 0;
+        CB_TRY(dbuf(c, "two_cs", T2 + To + (own ? T1 : 0), &dcs2));
+        if (old_too)
+            dcs = dcs2 + T2;
+        dpole = own ? dcs2 + T2 + To : dcs;
+    }
+    else
+        CB_TRY(dbuf(c, "cs", T1, &dcs));
     if (!in.dc)
     {
         CB_TRY(dbuf(c, "shc_in", (size_t)(2 * Ts), &raw));
@@ -1965,7 +1972,7 @@ Status shs_grid_run(Context &c, const charm_point *pnt, const CoefIn &in,
                                  c.stream), s2);
         if (with)
             G.pending = false;
-        if (dpole != dcs)
+        if (dpole && dpole != dcs)
         {
             S.cs = dpole;
             S.cs2 = nullptr;
@@ -2664,9 +2671,10 @@ Status shs_batch_run(Context &c, const charm_point *pnt, size_t nsets,
                                              (per_set + per_cs));
         bsz = std::min(bsz, nsets);
         if (two)
-            CB_TRY(dbuf(c, "two_batch_cs", bsz * (size_t)T2, &cs2_all));
+            CB_TRY(dbuf(c, "two_batch_cs",
+                        bsz * (size_t)(T2 + (old_too ? T : 0)), &cs2_all));
         if (two && old_too)
-            CB_TRY(dbuf(c, "two_batch_cs1", bsz * (size_t)T, &cs_all));
+            cs_all = cs2_all + bsz * (size_t)T2;
         double2 *lc = nullptr;
         CB_TRY(dbuf(c, "batch_lumped", bsz * per_set / sizeof(double2), &lc));
         BatchSet *dsets = nullptr;
@@ -3577,11 +3585,12 @@ Status sha_grid_run(Context &c, const charm_point *pnt, const double *f_host,
     int tpg = (int)((ntiles + Gn - 1) / Gn);
     Gn = (ntiles + tpg - 1) / tpg;
     double2 *part = nullptr, *part1 = nullptr;
-    CB_TRY(dbuf(c, "sha_part",
-                (size_t)Gn * (n2 > 0 ? 2 * two_sum((long long)nmax) : T),
-                &part));
-    if (n2 > 0 && n2 < np)
-        CB_TRY(dbuf(c, "sha_part1", (size_t)T, &part1));
+    const bool near = n2 > 0 && n2 < np;
+    const size_t Tp =
+        (size_t)Gn * (size_t)(n2 > 0 ? 2 * two_sum((long long)nmax) : T);
+    CB_TRY(dbuf(c, "sha_part", Tp + (near ? (size_t)T : 0), &part));
+    if (near)
+        part1 = part + Tp;
 
     // grid on the device and r2c along the parallels
     const double *fg = d_fin;
